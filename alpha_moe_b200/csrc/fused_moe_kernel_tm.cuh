@@ -151,7 +151,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     setmaxnreg_dec<40>();
     if (warp == W_MMA0 || warp == W_MMA0 + 1) {
         // ------------------------------------------------------------------ UMMA issuers (even / odd chunks)
-        if (lane == 0) {
+        {
             const int pw = warp - W_MMA0;
             constexpr uint32_t idesc256 = umma_idesc_e4m3(128, 256);
             constexpr uint32_t idesc128 = umma_idesc_e4m3(128, 128);
@@ -200,19 +200,22 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     if (!turn_ok) break;
                 }
                 if (!mbar_wait(&full[s], ph, abort_flag, p.status, 22, it)) break;
-                *issue_turn = it + 1;
-                fence_proxy_async_smem();      // token rows were written by cp.async, the UMMA reads them through the async proxy
                 tc_fence_after();
                 const uint64_t off = static_cast<uint64_t>(s * dstep);
-                if (up) {
-                    umma_f8_chunk1(d, x_0 + off, w_0 + off, idesc256);           // D[token, 256 interleaved w rows]
-                } else if (SPC == 1) {
-                    umma_f8_chunk1(d, h0, w_0 + off, idesc256);                  // D[token, 2 x 128 hidden rows]
-                } else {
-                    umma_f8_chunk2(d, d + 128, h0, h1, w_0 + off, w_1 + off, idesc128);   // per-slice partial sums
+                if (elect_one()) {
+                    *issue_turn = it + 1;
+                    fence_proxy_async_smem();  // token rows were written by cp.async, the UMMA reads them through the async proxy
+                    if (up) {
+                        umma_f8_chunk1(d, x_0 + off, w_0 + off, idesc256);           // D[token, 256 interleaved w rows]
+                    } else if (SPC == 1) {
+                        umma_f8_chunk1(d, h0, w_0 + off, idesc256);                  // D[token, 2 x 128 hidden rows]
+                    } else {
+                        umma_f8_chunk2(d, d + 128, h0, h1, w_0 + off, w_1 + off, idesc128);   // per-slice partial sums
+                    }
+                    umma_commit(&acc_full[b]);
+                    umma_commit(&empty[s]);    // the ring slot is free once these MMAs have read it
                 }
-                umma_commit(&acc_full[b]);
-                umma_commit(&empty[s]);        // the ring slot is free once these MMAs have read it
+                __syncwarp();
                 s += step;
                 while (s >= S) { s -= S; ph ^= 1; }
             }
