@@ -56,13 +56,6 @@ __host__ __device__ inline SmemPlanTm smem_plan_tm(int s, int kc, int spc) {
     return p;
 }
 
-__device__ __forceinline__ void red_add_v4_bf16x2_raw_if(__nv_bfloat16* addr, const uint4& w, bool pred) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
-        "@p red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};\n\t}"
-        ::"l"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(static_cast<uint32_t>(pred)));
-}
-
 constexpr int kTmThreads = 512;     // 2 epilogue warpgroups + control warpgroup + gather warpgroup
 constexpr int kTmGatherWarps = 5;   // one warp of the control warpgroup + the gather warpgroup
 

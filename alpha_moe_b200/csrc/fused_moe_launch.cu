@@ -667,6 +667,9 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     p.stages = depth;
     p.ksplit = ksplit;
     p.scaling = scaling_factor;
+    p.out_vec16 = 1;
+    for (int r = 0; r < tp_world; ++r)
+        if (reinterpret_cast<uintptr_t>(outs[r]) & 15) p.out_vec16 = 0;
     p.status = facts.status;
 
     const long long grid = nblocks * (N / 256 / spc) * ksplit;

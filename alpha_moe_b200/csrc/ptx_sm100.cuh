@@ -300,6 +300,56 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
 }
 __device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
+// The wait tied to the registers of the loads it completes: no use of them can be scheduled before it.
+__device__ __forceinline__ void tmem_ld_wait32(uint32_t (&a)[8], uint32_t (&b)[8], uint32_t (&c)[8], uint32_t (&d)[8]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(a[0]), "+r"(a[1]), "+r"(a[2]), "+r"(a[3]), "+r"(a[4]), "+r"(a[5]), "+r"(a[6]), "+r"(a[7]),
+                   "+r"(b[0]), "+r"(b[1]), "+r"(b[2]), "+r"(b[3]), "+r"(b[4]), "+r"(b[5]), "+r"(b[6]), "+r"(b[7]),
+                   "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3]), "+r"(c[4]), "+r"(c[5]), "+r"(c[6]), "+r"(c[7]),
+                   "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]), "+r"(d[4]), "+r"(d[5]), "+r"(d[6]), "+r"(d[7])
+                 :: "memory");
+}
+// 32 lanes x 16 columns as fragments (two 16-lane loads): v[h][4i], v[h][4i + 1] of thread t = lane 16h + t / 4, columns
+// 8i + 2 (t % 4) and the next; v[h][4i + 2], v[h][4i + 3] = the same columns of lane 16h + 8 + t / 4.
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_ld_frag16(uint32_t taddr, uint32_t (&v)[2][8]) {
+    tmem_ld_16x256b_x2(taddr, v[0]);
+    tmem_ld_16x256b_x2(taddr + (16u << 16), v[1]);
+}
+// Four 8 x 8 matrices of 16-bit values, stored transposed: thread t holds (row t / 4, columns 2 (t % 4) and the next)
+// of each; thread t's address is that of row t % 8 of transposed matrix t / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, const uint32_t (&m)[4]) {
+    asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};"
+                 ::"r"(addr), "r"(m[0]), "r"(m[1]), "r"(m[2]), "r"(m[3]) : "memory");
+}
+
+// --------------------------------------------------------------------------------------------- packed fp32 pairs
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack_u32x2(uint32_t lo, uint32_t hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+    return d;
+}
+__device__ __forceinline__ f32x2 pack_f32x2(float lo, float hi) { return pack_u32x2(__float_as_uint(lo), __float_as_uint(hi)); }
+__device__ __forceinline__ void unpack_f32x2(f32x2 d, float& lo, float& hi) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(d));
+}
+__device__ __forceinline__ f32x2 fma_f32x2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul_f32x2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+
 // --------------------------------------------------------------------------------------------- misc
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
@@ -317,6 +367,21 @@ __device__ __forceinline__ void red_add_bf16x2_if(__nv_bfloat16* addr, float lo,
         "{\n\t.reg .pred p;\n\tsetp.lt.s32 p, %2, %3;\n\t"
         "@p red.global.add.noftz.bf16x2 [%0], %1;\n\t}"
         ::"l"(addr), "r"(*reinterpret_cast<uint32_t*>(&v)), "r"(row), "r"(nrows));
+}
+// 16 bytes = 8 consecutive bf16 values in one reduction, issued only where `pred` holds.
+__device__ __forceinline__ void red_add_v4_bf16x2_raw_if(__nv_bfloat16* addr, const uint4& w, bool pred) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "@p red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};\n\t}"
+        ::"l"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(static_cast<uint32_t>(pred)));
+}
+// The same for an address that is only 4-byte aligned.
+__device__ __forceinline__ void red_add_4x_bf16x2_raw_if(__nv_bfloat16* addr, const uint4& w, bool pred) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
+        "@p red.global.add.noftz.bf16x2 [%0], %1;\n\t@p red.global.add.noftz.bf16x2 [%0 + 4], %2;\n\t"
+        "@p red.global.add.noftz.bf16x2 [%0 + 8], %3;\n\t@p red.global.add.noftz.bf16x2 [%0 + 12], %4;\n\t}"
+        ::"l"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(static_cast<uint32_t>(pred)));
 }
 // Register re-balancing between warpgroups (all four warps of a warpgroup must execute it).
 template <int N>

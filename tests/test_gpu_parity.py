@@ -95,6 +95,27 @@ def test_sixty_four_wide_blocks_two_ctas_per_sm(bm, bn, wn, stages):
     check_close(run_capi(case, bm, bn, wn, stages), orc.run_oracle(case, bm), tag=f"bm={bm} bn={bn} st={stages}")
 
 
+@pytest.mark.parametrize("bm,stages,m,k,inter", [
+    (24, 1, 70, 256, 256),       # one ring slot: the staging tile has its own memory
+    (32, 2, 333, 512, 512),      # two slice groups per block
+    (32, 5, 33, 128, 256),       # a single K chunk
+    (40, 2, 500, 384, 256),      # third column group half used
+    (48, 1, 190, 640, 256),
+    (56, 4, 400, 256, 256),      # two warpgroups, the second one partly used
+    (64, 2, 1, 256, 256),        # one live column
+    (64, 3, 17, 1152, 256),      # seventeen live columns: second column group of the first warpgroup
+])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_fragment_epilogue_edges(bm, stages, m, k, inter, offset):
+    """Tiles of 32 and 64 tokens with two slices per CTA: partly filled column groups, every ring depth class, and an
+    `out` that is only 4-byte aligned (offset in bf16 elements), which takes 4-byte reductions.  Bounds as above."""
+    case = orc.make_case(6, k, inter, m, 2, seed=bm + stages + m, scaling=1.5)
+    buf = torch.zeros(m * k + offset, dtype=torch.bfloat16, device="cuda:0")
+    out = buf[offset:].view(m, k)
+    check_close(run_capi(case, bm, 64, 4, stages, out=out), orc.run_oracle(case, bm), tag=f"bm={bm} st={stages} off={offset}")
+    assert not buf[:offset].any()
+
+
 def test_skewed_routing_with_empty_experts():
     """Zipf(1.2) routing: several experts receive nothing, a few receive >10% of the tokens, so the
     schedule has empty experts, multi-block experts and ragged padding."""
