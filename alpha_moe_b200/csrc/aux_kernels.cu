@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 
 #include "../../include/alpha_moe_b200.h"
@@ -173,68 +174,137 @@ moe_align_chunks_kernel(const int32_t* ids, int numel, int E, int block, int32_t
     scatter_chunk(ids, numel, chunk * kChunk, E, cnt, sorted);
 }
 
-// Everything in one CTA when there is a single chunk (numel <= kChunk: e.g. up to 113 tokens at top_k = 9).
-// cnt: 8 * kMaxExperts ints, warp_tot: 8 ints of shared memory.  Thread t owns the experts [t * per, (t + 1) * per):
-// their padded sizes, then (after a scan over the threads: warp shuffles and the eight warp totals) their first output
-// slots - a single thread walking over all experts took longer than everything else in this kernel together.
+// Everything in one CTA for up to kSingleMax assignments (227 tokens at top_k = 9).  Nothing here is more than a few
+// kilobytes; what counts is the number of dependent steps, so every load of an id is issued first, the default fills are
+// 16-byte stores, and there are three barriers.  Warp w owns 32 * rounds consecutive assignments; cnt[w][e] counts its
+// assignments of expert e, then (after thread t has turned the columns of its experts into exclusive sums over the
+// warps) it is the number of earlier ones, and start[e] the expert's first slot.
+// The line to the kernel with one CTA per 1024 assignments and a grid-wide barrier, in the call that also quantises (one
+// launch against two on two streams): 203 tokens (1827 assignments, 257 experts) 8.2 us against 10.7; 777 tokens (6993
+// assignments, with 16 rounds) 19.5 against 12.8 - match.any takes longer than a grid-wide barrier from about there on.
+// Few rounds also keep the code short, and at these sizes it is fetched cold: 1 token 4.1 -> 3.6 us, 24 tokens 6.4 -> 4.6,
+// 96 tokens at 512 experts 7.2 -> 6.2 (before: 256 threads, a serial walk of four rounds per warp).
+constexpr int kSingleThreads = 512;
+constexpr int kSingleWarps = kSingleThreads / 32;
+constexpr int kSingleRounds = 4;
+constexpr int kSingleMax = kSingleThreads * kSingleRounds;
+
+struct SingleSmem {
+    uint32_t cnt[kSingleWarps * kMaxExperts / 2];      // two 16-bit counters a word: kSingleMax fits 16 bits
+    int start[kMaxExperts];
+    int warp_tot[kSingleWarps];
+};
+
+__device__ __forceinline__ void fill_i32(int32_t* dst, int n, int32_t v) {
+    if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
+        const int4 q = make_int4(v, v, v, v);
+        for (int i = threadIdx.x; i < n / 4; i += kSingleThreads) reinterpret_cast<int4*>(dst)[i] = q;
+        for (int i = (n & ~3) + threadIdx.x; i < n; i += kSingleThreads) dst[i] = v;
+    } else {
+        for (int i = threadIdx.x; i < n; i += kSingleThreads) dst[i] = v;
+    }
+}
+
 __device__ __forceinline__ void align_single_body(const int32_t* ids, int numel, int E, int block, int32_t* sorted,
                                                   int sorted_len, int32_t* expert_ids, int n_blocks_max,
-                                                  int32_t* num_post_pad, int* cnt, int* warp_tot) {
-    for (int i = threadIdx.x; i < sorted_len; i += kAlignThreads) sorted[i] = numel;
-    for (int i = threadIdx.x; i < n_blocks_max; i += kAlignThreads) expert_ids[i] = 0;
-    count_chunk(ids, numel, 0, E, cnt);                   // (its barriers also order the default fills before the writes below)
-    const int per = (E + kAlignThreads - 1) / kAlignThreads;           // <= 4
-    int padded[4], mine = 0;
+                                                  int32_t* num_post_pad, SingleSmem& sm) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int rounds = (numel + kSingleThreads - 1) / kSingleThreads;         // <= kSingleRounds
+    const int p0 = warp * 32 * rounds + lane;
+    int id[kSingleRounds];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int r = 0; r < kSingleRounds; ++r) {
+        const int p = p0 + r * 32;
+        id[r] = r < rounds && p < numel ? ids[p] : -1;
+        if (id[r] < 0 || id[r] >= E) id[r] = -1;                              // ids outside [0,E) are ignored
+    }
+    for (int i = threadIdx.x; i < kSingleWarps * ((E + 1) / 2); i += kSingleThreads) sm.cnt[i] = 0;
+    fill_i32(sorted, sorted_len, numel);
+    fill_i32(expert_ids, n_blocks_max, 0);
+    __syncthreads();               // (also orders the default fills before the writes below)
+    const int row = (E + 1) & ~1;
+    uint16_t* cnt = reinterpret_cast<uint16_t*>(sm.cnt);
+    uint16_t* mine_cnt = cnt + warp * row;
+#pragma unroll
+    for (int r = 0; r < kSingleRounds; ++r) {
+        if (r < rounds) {
+            const unsigned same = __match_any_sync(0xFFFFFFFFu, id[r]);
+            if (id[r] >= 0 && (same & ((1u << lane) - 1)) == 0) mine_cnt[id[r]] += static_cast<uint16_t>(__popc(same));
+            __syncwarp();
+        }
+    }
+    __syncthreads();
+    const int live_warps = (numel + 32 * rounds - 1) / (32 * rounds);
+    const int per = (E + kSingleThreads - 1) / kSingleThreads;                // experts of a thread: one or two
+    int padded[2], mine = 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
         const int e = threadIdx.x * per + i;
         padded[i] = 0;
         if (i < per && e < E) {
             int tot = 0;
+            if (live_warps == 1) {
+                tot = cnt[e];
+                cnt[e] = 0;
+            } else {
+                uint16_t c[kSingleWarps];
 #pragma unroll
-            for (int w = 0; w < 8; ++w) tot += cnt[w * E + e];
+                for (int w = 0; w < kSingleWarps; ++w) c[w] = cnt[w * row + e];
+#pragma unroll
+                for (int w = 0; w < kSingleWarps; ++w) {
+                    cnt[w * row + e] = static_cast<uint16_t>(tot);
+                    tot += c[w];
+                }
+            }
             padded[i] = (tot + block - 1) / block * block;
             mine += padded[i];
         }
     }
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int incl = mine;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
         const int v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
         if (lane >= d) incl += v;
     }
-    if (lane == 31) warp_tot[warp] = incl;
+    if (lane == 31) sm.warp_tot[warp] = incl;
     __syncthreads();
     int run = incl - mine;
-    for (int w = 0; w < warp; ++w) run += warp_tot[w];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int w = 0; w < kSingleWarps; ++w) run += w < warp ? sm.warp_tot[w] : 0;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
         const int e = threadIdx.x * per + i;
         if (i < per && e < E) {
+            sm.start[e] = run;
             for (int b = run / block; b < (run + padded[i]) / block; ++b) expert_ids[b] = e;
-            int slot = run;
-#pragma unroll
-            for (int w = 0; w < 8; ++w) {          // counts -> first slot of each warp's assignments of expert e
-                const int n = cnt[w * E + e];
-                cnt[w * E + e] = slot;
-                slot += n;
-            }
             run += padded[i];
         }
     }
-    if (threadIdx.x == kAlignThreads - 1) num_post_pad[0] = run;       // the last thread's running end = total
+    if (threadIdx.x == kSingleThreads - 1) num_post_pad[0] = run;             // the last thread's running end = total
     __syncthreads();
-    scatter_chunk(ids, numel, 0, E, cnt, sorted);
+#pragma unroll
+    for (int r = 0; r < kSingleRounds; ++r) {
+        if (r < rounds) {
+            const unsigned same = __match_any_sync(0xFFFFFFFFu, id[r]);
+            const int leader = __ffs(same) - 1;
+            int before = 0;
+            if (id[r] >= 0 && lane == leader) {
+                before = mine_cnt[id[r]];
+                mine_cnt[id[r]] = static_cast<uint16_t>(before + __popc(same));
+            }
+            before = __shfl_sync(0xFFFFFFFFu, before, leader);
+            if (id[r] >= 0) sorted[sm.start[id[r]] + before + __popc(same & ((1u << lane) - 1))] = p0 + r * 32;
+            __syncwarp();
+        }
+    }
 }
 
-__global__ void __launch_bounds__(kAlignThreads)
+__global__ void __launch_bounds__(kSingleThreads, 2)
 moe_align_single_kernel(const int32_t* ids, int numel, int E, int block, int32_t* sorted, int sorted_len,
                         int32_t* expert_ids, int n_blocks_max, int32_t* num_post_pad) {
-    __shared__ int cnt[8 * kMaxExperts];
-    __shared__ int warp_tot[kAlignThreads / 32];
+    __shared__ SingleSmem sm;
     launch_dependents();
-    align_single_body(ids, numel, E, block, sorted, sorted_len, expert_ids, n_blocks_max, num_post_pad, cnt, warp_tot);
+    align_single_body(ids, numel, E, block, sorted, sorted_len, expert_ids, n_blocks_max, num_post_pad, sm);
 }
 
 // ------------------------------------------------------------------------------------------------
@@ -243,12 +313,13 @@ moe_align_single_kernel(const int32_t* ids, int numel, int E, int block, int32_t
 // 3 bytes per element, + 2 when the source is zeroed); a warp takes four consecutive groups per step and the grid
 // strides over the tensor.  The quotients are the correctly rounded IEEE ones, so the result is bit-identical to the
 // CPU restatement.
+template <int WARPS>
 __device__ __forceinline__ void group_quant_body(__nv_bfloat16* x, uint8_t* q, float* scale, long long n_groups,
                                                  int zero_src, int block, int nblocks) {
     const int lane = threadIdx.x & 31;
     const int sub = lane & 7;                   // 16-element piece of the group
-    const long long warp0 = static_cast<long long>(block) * 8 + (threadIdx.x >> 5);
-    const long long nwarps = static_cast<long long>(nblocks) * 8;
+    const long long warp0 = static_cast<long long>(block) * WARPS + (threadIdx.x >> 5);
+    const long long nwarps = static_cast<long long>(nblocks) * WARPS;
     // the loads of the next step are issued before the arithmetic of the current one (one step = 32 bytes per lane)
     uint4 n0 = make_uint4(0u, 0u, 0u, 0u), n1 = n0;
     {
@@ -325,26 +396,24 @@ __device__ __forceinline__ void group_quant_body(__nv_bfloat16* x, uint8_t* q, f
 __global__ void __launch_bounds__(256)
 group_quant_fp8_kernel(__nv_bfloat16* x, uint8_t* q, float* scale, long long n_groups, int zero_src) {
     launch_dependents();
-    group_quant_body(x, q, scale, n_groups, zero_src, blockIdx.x, gridDim.x);
+    group_quant_body<8>(x, q, scale, n_groups, zero_src, blockIdx.x, gridDim.x);
 }
 
 // The two steps in front of the operator at a serving call site - quantise the activations (and clear their buffer,
-// which the layer then accumulates into) and build the block schedule - are independent of each other.  For decode-
-// size batches, whose schedule fits one CTA, they run as one launch: the last CTA builds the schedule, the others
-// quantise.  Same code, same bits as the two separate kernels.
-__global__ void __launch_bounds__(256)
+// which the layer then accumulates into) and build the block schedule - are independent of each other.  Where the
+// schedule fits one CTA they run as one launch: the first CTA builds the schedule, the others quantise.  Same code, same
+// bits as the two separate kernels.
+__global__ void __launch_bounds__(kSingleThreads, 2)
 quant_and_align_small_kernel(__nv_bfloat16* x, uint8_t* q, float* scale, long long n_groups, int zero_src,
                              const int32_t* ids, int numel, int E, int block, int32_t* sorted, int sorted_len,
                              int32_t* expert_ids, int n_blocks_max, int32_t* num_post_pad) {
-    __shared__ int cnt[8 * kMaxExperts];
-    __shared__ int warp_tot[kAlignThreads / 32];
-    static_assert(kAlignThreads == 256, "one block shape for both halves");
+    __shared__ SingleSmem sm;
     launch_dependents();      // the operator behind this launch may be scheduled; it waits for our completion
-    if (blockIdx.x == gridDim.x - 1) {
-        align_single_body(ids, numel, E, block, sorted, sorted_len, expert_ids, n_blocks_max, num_post_pad, cnt, warp_tot);
+    if (blockIdx.x == 0) {
+        align_single_body(ids, numel, E, block, sorted, sorted_len, expert_ids, n_blocks_max, num_post_pad, sm);
         return;
     }
-    group_quant_body(x, q, scale, n_groups, zero_src, blockIdx.x, gridDim.x - 1);
+    group_quant_body<kSingleWarps>(x, q, scale, n_groups, zero_src, blockIdx.x - 1, gridDim.x - 1);
 }
 
 // Scratch of the entry point that allocates nothing: the per-chunk histogram table lives here instead of
@@ -401,14 +470,14 @@ int alpha_moe_b200_moe_align_block_size(const int32_t* topk_ids, int numel, int 
     const int n_blocks_max = static_cast<int>((sorted_len + block_m - 1) / block_m);
     const int chunks = (numel + kChunk - 1) / kChunk;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    if (chunks == 1) {
-        moe_align_single_kernel<<<1, kAlignThreads, 0, st>>>(topk_ids, numel, num_experts, block_m, sorted_token_ids,
+    if (chunks > 1 && !workspace) return fail(ALPHA_MOE_E_ARG, "workspace is required for more than %d assignments", kChunk);
+    if (numel <= kSingleMax) {
+        moe_align_single_kernel<<<1, kSingleThreads, 0, st>>>(topk_ids, numel, num_experts, block_m, sorted_token_ids,
                                                             static_cast<int>(sorted_len), expert_ids, n_blocks_max,
                                                             num_tokens_post_padded);
         AUX_TRY(cudaGetLastError());
         return ALPHA_MOE_OK;
     }
-    if (!workspace) return fail(ALPHA_MOE_E_ARG, "workspace is required for more than %d assignments", kChunk);
     int* hist = static_cast<int*>(workspace);
     int sorted_len_i = static_cast<int>(sorted_len);
     int n_blocks_max_v = n_blocks_max, numel_v = numel, e_v = num_experts, block_v = block_m;
@@ -510,7 +579,7 @@ int alpha_moe_b200_quant_and_align(void* x_bf16, void* x_fp8, float* x_scale, in
     if (num_experts <= 0 || num_experts > kMaxExperts)
         return fail(ALPHA_MOE_E_ARG, "num_experts must be in 1..%d (got %d)", kMaxExperts, num_experts);
     if (block_m <= 0) return fail(ALPHA_MOE_E_ARG, "block_m must be positive (got %d)", block_m);
-    if (numel > kChunk) {
+    if (numel > kSingleMax) {
         // Two launches (the schedule needs several CTAs and a grid-wide barrier) that do not depend on each other: the
         // schedule runs on a side stream forked from the caller's and joined back into it, beside the quantiser.  It
         // is launched first so that its few CTAs have their places before the quantiser's grid fills every SM.
@@ -531,12 +600,17 @@ int alpha_moe_b200_quant_and_align(void* x_bf16, void* x_fp8, float* x_scale, in
         }
         return rc_quant;
     }
+    if (numel > kChunk && !workspace) return fail(ALPHA_MOE_E_ARG, "workspace is required for more than %d assignments", kChunk);
     const long long sorted_len = numel + static_cast<long long>(num_experts) * (block_m - 1);
     if (sorted_len > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "schedule too long for int32 indices");
     const int n_blocks_max = static_cast<int>((sorted_len + block_m - 1) / block_m);
     const long long n_groups = static_cast<long long>(M) * (K / 128);
-    const long long qblocks = (n_groups + 31) / 32;      // at most 1024 * K / 4096 blocks: no cap needed
-    quant_and_align_small_kernel<<<static_cast<unsigned>(qblocks + 1), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    // a warp takes four groups per step; beyond 16 steps' worth of warps per SM the rest is covered by the stride
+    int dev = 0, sms = 0;
+    AUX_TRY(cudaGetDevice(&dev));
+    AUX_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    const long long qblocks = std::min<long long>((n_groups + 4 * kSingleWarps - 1) / (4 * kSingleWarps), 4LL * sms);
+    quant_and_align_small_kernel<<<static_cast<unsigned>(qblocks + 1), kSingleThreads, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<__nv_bfloat16*>(x_bf16), static_cast<uint8_t*>(x_fp8), x_scale, n_groups, zero_src, topk_ids,
         static_cast<int>(numel), num_experts, block_m, sorted_token_ids, static_cast<int>(sorted_len), expert_ids,
         n_blocks_max, num_tokens_post_padded);
