@@ -4,6 +4,7 @@ layer accumulates into, block schedule, fused operator.  `hidden_states` holds t
 as in the patch.  Buffers come from torch; the work is one C-ABI call."""
 from __future__ import annotations
 
+import contextlib
 import os
 
 import torch
@@ -12,36 +13,51 @@ from . import capi
 from .utils import get_best_config
 
 
+def _up(n: int) -> int:
+    return (n + 255) & ~255
+
+
 def _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids) -> None:
     """The checks the torch operator makes on its tensors (csrc/torch_interface.cpp:58-76 of the reference, plus
     the dtype / device / shape checks this library's operator adds), made here before any raw pointer is taken:
     this path goes straight to the C ABI, which sees only addresses."""
-    def need(cond, msg):
-        if not cond:
-            raise RuntimeError(msg)
-    need(hidden_states.dtype == torch.bfloat16 and hidden_states.dim() == 2 and hidden_states.is_contiguous(),
-         "hidden_states must be a contiguous 2-D bfloat16 tensor")
+    # (written out: messages are only put together for a call that fails)
+    if hidden_states.dtype != torch.bfloat16 or hidden_states.dim() != 2 or not hidden_states.is_contiguous():
+        raise RuntimeError("hidden_states must be a contiguous 2-D bfloat16 tensor")
     dev = hidden_states.device
     m, k = hidden_states.shape
-    need(m > 0, "hidden_states must have at least one row")
-    need(k % 128 == 0, "K dimension must be a multiple of 128")
-    need(w1.dim() == 3 and w2.dim() == 3, "w1 must be [E, 2I, K] and w2 [E, K, I]")
+    if m <= 0:
+        raise RuntimeError("hidden_states must have at least one row")
+    if k % 128 != 0:
+        raise RuntimeError("K dimension must be a multiple of 128")
+    if w1.dim() != 3 or w2.dim() != 3:
+        raise RuntimeError("w1 must be [E, 2I, K] and w2 [E, K, I]")
     e, n, kw = w1.shape
-    need(kw == k, "w1.size(2) must equal hidden_states.size(1)")
-    need(n % 256 == 0, "N (2 x intermediate size) must be a multiple of 256")
-    need(tuple(w2.shape) == (e, k, n // 2), "w2 must be [E, K, N/2]")
-    need(w1.dtype == torch.float8_e4m3fn and w2.dtype == torch.float8_e4m3fn, "w1 and w2 must be float8_e4m3fn")
-    need(tuple(w1_scale.shape) == (e, n // 128, k // 128), "w1_scale must be [E, N/128, K/128]")
-    need(tuple(w2_scale.shape) == (e, k // 128, n // 256), "w2_scale must be [E, K/128, N/256]")
-    need(w1_scale.dtype == torch.float32 and w2_scale.dtype == torch.float32, "weight scales must be float32")
-    need(topk_ids.dim() == 2 and topk_ids.shape[0] == m, "topk_ids must be [M, top_k]")
-    need(tuple(topk_weights.shape) == tuple(topk_ids.shape), "topk_weights must have the shape of topk_ids")
-    for name, t in (("w1", w1), ("w1_scale", w1_scale), ("w2", w2), ("w2_scale", w2_scale)):
-        need(t.is_contiguous(), f"{name} must be contiguous")
-    for name, t in (("w1", w1), ("w1_scale", w1_scale), ("w2", w2), ("w2_scale", w2_scale),
-                    ("topk_weights", topk_weights), ("topk_ids", topk_ids)):
-        need(t.device == dev, f"{name} must be on {dev}")
-
+    if kw != k:
+        raise RuntimeError("w1.size(2) must equal hidden_states.size(1)")
+    if n % 256 != 0:
+        raise RuntimeError("N (2 x intermediate size) must be a multiple of 256")
+    if w2.shape != (e, k, n // 2):
+        raise RuntimeError("w2 must be [E, K, N/2]")
+    if w1.dtype != torch.float8_e4m3fn or w2.dtype != torch.float8_e4m3fn:
+        raise RuntimeError("w1 and w2 must be float8_e4m3fn")
+    if w1_scale.shape != (e, n // 128, k // 128):
+        raise RuntimeError("w1_scale must be [E, N/128, K/128]")
+    if w2_scale.shape != (e, k // 128, n // 256):
+        raise RuntimeError("w2_scale must be [E, K/128, N/256]")
+    if w1_scale.dtype != torch.float32 or w2_scale.dtype != torch.float32:
+        raise RuntimeError("weight scales must be float32")
+    if topk_ids.dim() != 2 or topk_ids.shape[0] != m:
+        raise RuntimeError("topk_ids must be [M, top_k]")
+    if topk_weights.shape != topk_ids.shape:
+        raise RuntimeError("topk_weights must have the shape of topk_ids")
+    weights = (w1, w1_scale, w2, w2_scale)
+    for i, t in enumerate(weights):
+        if not t.is_contiguous():
+            raise RuntimeError(f"{('w1', 'w1_scale', 'w2', 'w2_scale')[i]} must be contiguous")
+    for i, t in enumerate((*weights, topk_weights, topk_ids)):
+        if t.device != dev:
+            raise RuntimeError(f"{('w1', 'w1_scale', 'w2', 'w2_scale', 'topk_weights', 'topk_ids')[i]} must be on {dev}")
 
 def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: torch.Tensor, w2: torch.Tensor,
                        w2_scale: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,
@@ -67,21 +83,29 @@ def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: 
         conf = get_best_config(path, m)
     block_m, bn, wn, stages = conf["block_m"], conf["block_n"], conf["warp_n"], conf["stages"]
     dev = hidden_states.device
-    ids = topk_ids.to(torch.int32).contiguous()
-    wts = topk_weights.to(torch.float32).contiguous()
+    ids = topk_ids if topk_ids.dtype == torch.int32 and topk_ids.is_contiguous() else topk_ids.to(torch.int32).contiguous()
+    wts = (topk_weights if topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
+           else topk_weights.to(torch.float32).contiguous())
+    # One allocation holds every intermediate buffer (256-byte aligned pieces); at one token the call is bound by its
+    # host time, and seven allocations were a third of it.
     numel = m * top_k
     total = numel + e * (block_m - 1)
-    x_q = torch.empty(m, k, dtype=torch.float8_e4m3fn, device=dev)
-    x_s = torch.empty(m, k // 128, dtype=torch.float32, device=dev)
-    sorted_ids = torch.empty(total, dtype=torch.int32, device=dev)
-    expert_ids = torch.empty((total + block_m - 1) // block_m, dtype=torch.int32, device=dev)
-    num_post_pad = torch.empty(1, dtype=torch.int32, device=dev)
     ws_bytes = capi.align_workspace_bytes(numel, e)
-    ws = torch.empty(max(ws_bytes, 4), dtype=torch.uint8, device=dev)
-    with torch.cuda.device(dev):
-        capi.fused_experts(hidden_states.data_ptr(), x_q.data_ptr(), x_s.data_ptr(), w1.data_ptr(), w1_scale.data_ptr(),
+    x_s = _up(m * k)
+    sorted_ids = x_s + _up(m * (k // 128) * 4)
+    expert_ids = sorted_ids + _up(total * 4)
+    num_post_pad = expert_ids + _up((total + block_m - 1) // block_m * 4)
+    ws = num_post_pad + 256
+    buf = torch.empty(ws + ws_bytes, dtype=torch.uint8, device=dev)
+    base = buf.data_ptr()
+    if dev.index == torch.cuda.current_device():
+        on_device = contextlib.nullcontext()
+    else:
+        on_device = torch.cuda.device(dev)
+    with on_device:
+        capi.fused_experts(hidden_states.data_ptr(), base, base + x_s, w1.data_ptr(), w1_scale.data_ptr(),
                            w2.data_ptr(), w2_scale.data_ptr(), ids.data_ptr(), wts.data_ptr(), top_k, m, k, n, e,
-                           sorted_ids.data_ptr(), expert_ids.data_ptr(), num_post_pad.data_ptr(),
-                           ws.data_ptr() if ws_bytes else 0, block_m, bn, wn, stages,
-                           float(routed_scaling_factor or 1.0), torch.cuda.current_stream(dev).cuda_stream)
+                           base + sorted_ids, base + expert_ids, base + num_post_pad, base + ws if ws_bytes else 0,
+                           block_m, bn, wn, stages, float(routed_scaling_factor or 1.0),
+                           torch._C._cuda_getCurrentRawStream(dev.index))
     return hidden_states
