@@ -349,24 +349,30 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const int b = it & 1;
             const uint32_t aph = (it >> 1) & 1;
             const float sx = xs[kc * kTmRows + t];
+            const float fg = sx * swg[sl * KC + kc], fu = sx * swu[sl * KC + kc];
             if (!mbar_wait(&acc_full[b], aph, abort_flag, p.status, 40, it)) { ok = false; break; }
             tc_fence_after();
             if (warp_valid) {
-                const float fg = sx * swg[sl * KC + kc], fu = sx * swu[sl * KC + kc];
                 const uint32_t tb = tlane + b * 256 + hh * 128;
+                // 64 columns are requested before the first is used (every wait lengthens the chain issue -> read-back ->
+                // hand-back around the two accumulator buffers): against waits after every 32 columns, blocks of 128 at
+                // the DeepSeek-V3 TP8 shard, M = 4096 460 -> 449 us, M = 8192 (Zipf) 769 -> 754 us, unsharded M = 4096
+                // 3540 -> 3212 us.  TMEM loads do not wait for UMMAs in flight: 16 columns and their FMAs take 40 cycles
+                // either way.
 #pragma unroll
-                for (int c0 = 0; c0 < 128; c0 += 32) {
-                    uint32_t va[16], vb[16];
-                    tmem_ld16(tb + c0, va);
-                    tmem_ld16(tb + c0 + 16, vb);
+                for (int c0 = 0; c0 < 128; c0 += 64) {
+                    uint32_t v[4][16];
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) tmem_ld16(tb + c0 + 16 * c, v[c]);
                     tmem_ld_wait();
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        acc[c0 + e] = fmaf(__uint_as_float(va[e]), fg, acc[c0 + e]);
-                        acc[c0 + 8 + e] = fmaf(__uint_as_float(va[8 + e]), fu, acc[c0 + 8 + e]);
-                        acc[c0 + 16 + e] = fmaf(__uint_as_float(vb[e]), fg, acc[c0 + 16 + e]);
-                        acc[c0 + 24 + e] = fmaf(__uint_as_float(vb[8 + e]), fu, acc[c0 + 24 + e]);
-                    }
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const int j = c0 + 16 * c + e;
+                            acc[j] = fmaf(__uint_as_float(v[c][e]), fg, acc[j]);
+                            acc[j + 8] = fmaf(__uint_as_float(v[c][8 + e]), fu, acc[j + 8]);
+                        }
                 }
             }
             tc_fence_before();
