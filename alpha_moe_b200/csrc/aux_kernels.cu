@@ -40,8 +40,8 @@ using amoe_capi::fail;
 //   phase C  stable scatter: warps walk their 128 assignments in order, ranking equal experts inside a warp round
 //            with match.any
 // One launch runs all three phases with a grid-wide barrier after phase A (a cooperative launch, used whenever all
-// chunks fit on the GPU at once); otherwise phase A and phases B + C are two launches of the same kernel.  When
-// everything fits one chunk the phases run inside one CTA of an ordinary launch.
+// chunks fit on the GPU at once); otherwise phase A and phases B + C are two launches of the same kernel.  Up
+// to kSingleMax assignments are the work of one CTA of an ordinary launch (align_single_body).
 // Programmatic dependent launch: the kernel behind this one in the stream (the fused operator, which is launched with
 // the matching attribute and waits for this kernel's completion before it reads anything) may be scheduled from here on.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
