@@ -54,6 +54,8 @@ lib.alpha_moe_b200_fused_experts.argtypes = [_vp] * 9 + [_i] * 5 + [_vp] * 4 + [
 lib.alpha_moe_b200_fused_experts.restype = _i
 lib.alpha_moe_b200_selftest_wait_timeout.restype = _i
 lib.alpha_moe_b200_selftest_wait_timeout.argtypes = [_i, _i, _i, _vp, _vp]
+lib.alpha_moe_b200_selftest_warp_wait.restype = _i
+lib.alpha_moe_b200_selftest_warp_wait.argtypes = [_i, _vp, _vp]
 lib.alpha_moe_b200_last_error.restype = ctypes.c_char_p
 lib.alpha_moe_b200_version.restype = ctypes.c_char_p
 
@@ -166,6 +168,11 @@ def fused_experts(hidden_states, x_fp8, x_scale, w, w_scale, w2, w2_scale, topk_
 def selftest_wait_timeout(limit_cycles: int, where: int, iter_: int, result2, stream=0) -> None:
     """Launches the bounded-wait self-test; result2 = device address of two int32 (what the two waits returned)."""
     _check(lib.alpha_moe_b200_selftest_wait_timeout(limit_cycles, where, iter_, result2, stream))
+
+
+def selftest_warp_wait(limit_cycles: int, result5, stream=0) -> None:
+    """Launches the self-test of the whole-warp waits; result5 = device address of five int32 (ballots of the answers)."""
+    _check(lib.alpha_moe_b200_selftest_warp_wait(limit_cycles, result5, stream))
 
 
 def read_status(reset: bool = False):

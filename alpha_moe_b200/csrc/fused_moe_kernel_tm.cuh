@@ -165,34 +165,17 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                 const uint32_t d = tmem_base + b * 256;
                 const bool up = it < UPI;
                 if (!up && !h_waited) {
-                    if (!mbar_wait(h_ready, 0, abort_flag, p.status, 20, it)) break;
+                    if (!mbar_wait_warp(h_ready, 0, abort_flag, p.status, 20, it)) break;
                     h_waited = true;
                 }
-                if (!mbar_wait(&acc_empty[b], aph ^ 1, abort_flag, p.status, 21, it)) break;
+                if (!mbar_wait_warp(&acc_empty[b], aph ^ 1, abort_flag, p.status, 21, it)) break;
                 // The two issuers take their turns in iteration order.  A parity wait is only meaningful while
                 // the waiter is at most one phase ahead of the barrier: waiting for fill n of a slot presumes
                 // that fill n-1 has completed.  Fill n-1 belongs to iteration it-S, which with an odd ring depth
                 // is the other issuer's; in the down phase the two warpgroups of the epilogue release the
                 // accumulator buffers independently, so without the turn one issuer could get that far ahead.
-                {
-                    const long long t0 = clock64();
-                    bool turn_ok = true;
-                    while (*issue_turn < it) {
-                        if (*abort_flag) { turn_ok = false; break; }
-                        if (clock64() - t0 > kWaitLimitCycles) {
-                            *abort_flag = 1;
-                            if (atomicCAS(&p.status->code, ST_OK, ST_WAIT_TIMEOUT) == ST_OK) {
-                                p.status->block = blockIdx.x;
-                                p.status->where = 23;
-                                p.status->iter = it;
-                            }
-                            turn_ok = false;
-                            break;
-                        }
-                    }
-                    if (!turn_ok) break;
-                }
-                if (!mbar_wait(&full[s], ph, abort_flag, p.status, 22, it)) break;
+                if (!turn_wait_warp(issue_turn, it, abort_flag, p.status, 23)) break;
+                if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, 22, it)) break;
                 tc_fence_after();
                 const uint64_t off = static_cast<uint64_t>(s * dstep);
                 if (elect_one()) {

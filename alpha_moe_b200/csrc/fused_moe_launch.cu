@@ -315,6 +315,37 @@ __global__ void wait_selftest_kernel(amoe::KernelStatus* status, int* result, lo
     }
 }
 
+// Self-test of the whole-warp waits with lanes that see different things: whatever each lane saw, all 32 must return the
+// same answer.  result[i] = ballot of the answers of
+//   0  lanes 0-15 wait on a completed mbarrier, 16-31 on one that never completes    1  all on the completed one
+//   2  lanes 0-15 see a turn that has come, 16-31 one that never does                3  all see the one that has come
+//   4  nothing completes, the abort flag is raised for lanes 0-15 only (no wait for the limit)
+__global__ void warp_wait_selftest_kernel(amoe::KernelStatus* status, unsigned* result, long long limit_cycles) {
+    __shared__ uint64_t bars[2];                   // never completed, completed
+    __shared__ int abort_flags[5], turns[2];
+    if (threadIdx.x == 0) {
+        amoe::mbar_init(&bars[0], 1);
+        amoe::mbar_init(&bars[1], 1);
+        for (int i = 0; i < 5; ++i) abort_flags[i] = i == 3;
+        turns[0] = 0;
+        turns[1] = 5;
+        amoe::fence_mbar_init();
+        amoe::mbar_arrive(&bars[1]);
+    }
+    __syncwarp();
+    const int split = threadIdx.x < 16;
+    const bool answer[5] = {
+        amoe::mbar_wait_warp_limit(&bars[split], 0, &abort_flags[0], status, 50, 0, limit_cycles),
+        amoe::mbar_wait_warp_limit(&bars[1], 0, &abort_flags[2], status, 51, 1, limit_cycles),
+        amoe::turn_wait_warp_limit(&turns[split], 5, &abort_flags[1], status, 52, limit_cycles),
+        amoe::turn_wait_warp_limit(&turns[1], 5, &abort_flags[2], status, 53, limit_cycles),
+        amoe::mbar_wait_warp(&bars[0], 0, &abort_flags[split ? 3 : 4], status, 54, 4)};
+    for (int i = 0; i < 5; ++i) {
+        const unsigned b = __ballot_sync(0xFFFFFFFFu, answer[i]);
+        if (threadIdx.x == 0) result[i] = b;
+    }
+}
+
 std::atomic<int> g_ksplit_override{0};     // 0 = automatic; set through alpha_moe_b200_set_ksplit (tuners, tests)
 
 // Clusters of CTAs along K for small batches (narrow tile, one slice per CTA only): the largest cluster size for
@@ -853,6 +884,20 @@ int alpha_moe_b200_selftest_wait_timeout(int limit_cycles, int where, int iter, 
     DeviceFacts facts;
     if (int rc = device_facts(dev, &facts)) return rc;
     wait_selftest_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(facts.status, result2, limit_cycles, where, iter);
+    CUDA_TRY(cudaGetLastError());
+    return ALPHA_MOE_OK;
+}
+
+int alpha_moe_b200_selftest_warp_wait(int limit_cycles, int32_t* result5, void* stream) {
+    if (!result5) return fail(ALPHA_MOE_E_ARG, "result5 is null");
+    if (limit_cycles < 1000 || limit_cycles > 200000000)
+        return fail(ALPHA_MOE_E_ARG, "limit_cycles must be in 1000..200000000 (about 0.1 s), got %d", limit_cycles);
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    DeviceFacts facts;
+    if (int rc = device_facts(dev, &facts)) return rc;
+    warp_wait_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(facts.status, reinterpret_cast<unsigned*>(result5),
+                                                                            limit_cycles);
     CUDA_TRY(cudaGetLastError());
     return ALPHA_MOE_OK;
 }

@@ -69,10 +69,21 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // Limit of one wait, in SM clock cycles (about a second at B200 clocks).
 constexpr long long kWaitLimitCycles = 2000000000LL;
 
+// First wait of a launch to run out: raises the CTA's abort flag and records where it was.
+__device__ __forceinline__ void record_run_out(volatile int* abort_flag, KernelStatus* status, int where, int iter) {
+    *abort_flag = 1;
+    if (atomicCAS(&status->code, ST_OK, ST_WAIT_TIMEOUT) == ST_OK) {
+        status->block = blockIdx.x;
+        status->where = where;
+        status->iter = iter;
+    }
+}
+
 // Bounded wait.  `abort_flag` is a CTA-shared word: once any thread of the CTA gives up, every
 // other waiter of that CTA returns false at its next poll, so the CTA unwinds as a whole.
 // (Kept inline: a device function call inside a role that has resized its register allotment with
 // setmaxnreg does not get through register allocation.)
+// Each thread decides for itself: for a single lane, or for threads that need no other lane afterwards.
 __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                                 KernelStatus* status, int where, int iter, long long limit_cycles) {
     if (mbar_try_wait(bar, parity)) return true;
@@ -83,12 +94,7 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
             if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > limit_cycles) {
-            *abort_flag = 1;
-            if (atomicCAS(&status->code, ST_OK, ST_WAIT_TIMEOUT) == ST_OK) {
-                status->block = blockIdx.x;
-                status->where = where;
-                status->iter = iter;
-            }
+            record_run_out(abort_flag, status, where, iter);
             return false;
         }
     }
@@ -96,6 +102,45 @@ __device__ __forceinline__ bool mbar_wait_limit(uint64_t* bar, uint32_t parity, 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           KernelStatus* status, int where, int iter) {
     return mbar_wait_limit(bar, parity, abort_flag, status, where, iter, kWaitLimitCycles);
+}
+
+// The same for a whole warp whose next steps need all 32 lanes (elect.sync, __syncwarp): the lanes vote on every poll, so
+// all of them get the same answer by construction.  With a decision per lane, one that gives up (the abort flag, its own
+// clock) while another has seen the barrier complete would leave the other at the next full-mask instruction for good.
+__device__ __forceinline__ bool mbar_wait_warp_limit(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                                     KernelStatus* status, int where, int iter, long long limit_cycles) {
+    if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 32; ++i)
+            if (__all_sync(0xFFFFFFFFu, mbar_try_wait(bar, parity))) return true;
+        const bool run_out = clock64() - t0 > limit_cycles;
+        if (run_out) record_run_out(abort_flag, status, where, iter);
+        if (__any_sync(0xFFFFFFFFu, run_out || *abort_flag != 0)) return false;
+    }
+}
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
+                                               KernelStatus* status, int where, int iter) {
+    return mbar_wait_warp_limit(bar, parity, abort_flag, status, where, iter, kWaitLimitCycles);
+}
+// A whole warp waits until the counter `turn` in shared memory has reached `it`; one answer for all lanes, as above.
+__device__ __forceinline__ bool turn_wait_warp_limit(volatile int* turn, int it, volatile int* abort_flag,
+                                                     KernelStatus* status, int where, long long limit_cycles) {
+    if (__all_sync(0xFFFFFFFFu, *turn >= it)) return true;
+    const long long t0 = clock64();
+    for (;;) {
+#pragma unroll 1
+        for (int i = 0; i < 8; ++i)
+            if (__all_sync(0xFFFFFFFFu, *turn >= it)) return true;
+        const bool run_out = clock64() - t0 > limit_cycles;
+        if (run_out) record_run_out(abort_flag, status, where, it);
+        if (__any_sync(0xFFFFFFFFu, run_out || *abort_flag != 0)) return false;
+    }
+}
+__device__ __forceinline__ bool turn_wait_warp(volatile int* turn, int it, volatile int* abort_flag, KernelStatus* status,
+                                               int where) {
+    return turn_wait_warp_limit(turn, it, abort_flag, status, where, kWaitLimitCycles);
 }
 
 // --------------------------------------------------------------------------------------------- clusters / DSMEM
@@ -145,12 +190,7 @@ __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity
             if (mbar_try_wait_cluster(bar, parity)) return true;
         if (*abort_flag) return false;
         if (clock64() - t0 > kWaitLimitCycles) {
-            *abort_flag = 1;
-            if (atomicCAS(&status->code, ST_OK, ST_WAIT_TIMEOUT) == ST_OK) {
-                status->block = blockIdx.x;
-                status->where = where;
-                status->iter = iter;
-            }
+            record_run_out(abort_flag, status, where, iter);
             return false;
         }
     }

@@ -186,6 +186,12 @@ int alpha_moe_b200_read_status(int32_t* out4, int reset);
  * with alpha_moe_b200_read_status afterwards (and clear it).  limit_cycles in 1000..200000000. */
 int alpha_moe_b200_selftest_wait_timeout(int limit_cycles, int where, int iter, int32_t* result2, void* stream);
 
+/* Self-test of the waits made by a whole warp (the threads that issue the matrix instructions), whose lanes must all
+ * get the same answer: one warp waits with lanes that see different barriers, turns or abort flags.  result5 (device, 5 x
+ * int32) receives the ballots of the answers: {0, ~0, 0, ~0, 0}.  Two of the waits run out after `limit_cycles` SM clocks
+ * (1000..200000000), so the status word is set as above (where = 50); the kernel returns normally. */
+int alpha_moe_b200_selftest_warp_wait(int limit_cycles, int32_t* result5, void* stream);
+
 /* What the launcher uses for a problem and a knob tuple; for tuners and tests.  It runs the launcher's own
  * planning code.  num_blocks = live upper bound of schedule blocks, min(ceil(sorted_num / block_m), M * top_k);
  * num_sms = SM count of a device (148 on B200): the cluster capacity that decides ksplit is then modelled (GPCs of

@@ -40,6 +40,18 @@ def test_selftest_rejects_limits_that_would_stall_the_gpu():
         capi.selftest_wait_timeout(10000, 1, 1, 0)
 
 
+def test_lanes_that_see_different_things_still_get_one_answer():
+    """The warps that issue the matrix instructions wait as whole warps and then need all 32 lanes (elect.sync,
+    __syncwarp).  Lanes that see different barriers, turns or abort flags must leave the wait together."""
+    from alpha_moe_b200 import capi
+    assert capi.read_status(reset=True)[0] == 0
+    res = torch.full((5,), 7, dtype=torch.int32, device="cuda")
+    capi.selftest_warp_wait(200_000, res.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert res.tolist() == [0, -1, 0, -1, 0]
+    assert capi.read_status(reset=True) == (1, 0, 50, 0)          # the first wait to run out is the one on record
+
+
 @pytest.mark.parametrize("which", ["barrier", "exchange_sum", "allreduce", "reduce_scatter"])
 def test_cross_gpu_wait_runs_out_when_a_rank_never_arrives(which):
     """The tensor-parallel exchange kernels wait for the other ranks through flag words in peer-mapped memory.  Here
