@@ -200,13 +200,20 @@ int launch_dependent(Kern kern, int grid, int threads, int smem_bytes, int clust
     return ALPHA_MOE_OK;
 }
 
-template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false>
+template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false, bool GENERAL = false>
 int launch_variant(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
-    auto kern = amoe::fused_moe_w8a8_up_down_sm100_kernel<BMP, SPC, EW, PEERS>;
+    auto kern = amoe::fused_moe_w8a8_up_down_sm100_kernel<BMP, SPC, EW, PEERS, GENERAL>;
     static std::atomic<int> configured[kMaxDevices];
     if (int rc = ensure_smem_attr(kern, configured, dev)) return rc;
     constexpr int threads = 128 * EW + 128;
     return launch_dependent(kern, grid, threads, smem_bytes, p.ksplit, stream, maps, p);
+}
+
+// A shape with the fragment epilogue: a ring of one slot takes its general form (see the kernel).
+template <int BMP, int EW, bool PEERS>
+int launch_frag(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
+    return p.stages == 1 ? launch_variant<BMP, 2, EW, PEERS, true>(maps, p, grid, smem_bytes, dev, stream)
+                         : launch_variant<BMP, 2, EW, PEERS, false>(maps, p, grid, smem_bytes, dev, stream);
 }
 
 template <int SPC>
@@ -723,8 +730,8 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
         }
         switch (bmp) {
             case 16: return launch_variant<16, 2, 1, true>(maps, p, g, smem_bytes, dev, st);
-            case 32: return launch_variant<32, 2, 1, true>(maps, p, g, smem_bytes, dev, st);
-            default: return launch_variant<64, 2, 2, true>(maps, p, g, smem_bytes, dev, st);
+            case 32: return launch_frag<32, 1, true>(maps, p, g, smem_bytes, dev, st);
+            default: return launch_frag<64, 2, true>(maps, p, g, smem_bytes, dev, st);
         }
     }
     if (spc == 1) {
@@ -737,9 +744,9 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     }
     switch (bmp) {
         case 16: return launch_variant<16, 2>(maps, p, g, smem_bytes, dev, st);
-        case 32: return launch_variant<32, 2>(maps, p, g, smem_bytes, dev, st);
-        default: return pair64 ? launch_variant<64, 2, 1>(maps, p, g, smem_bytes, dev, st)
-                               : launch_variant<64, 2>(maps, p, g, smem_bytes, dev, st);
+        case 32: return launch_frag<32, 1, false>(maps, p, g, smem_bytes, dev, st);
+        default: return pair64 ? launch_frag<64, 1, false>(maps, p, g, smem_bytes, dev, st)
+                               : launch_frag<64, 2, false>(maps, p, g, smem_bytes, dev, st);
     }
 }
 

@@ -96,7 +96,8 @@ def test_sixty_four_wide_blocks_two_ctas_per_sm(bm, bn, wn, stages):
 
 
 @pytest.mark.parametrize("bm,stages,m,k,inter", [
-    (24, 1, 70, 256, 256),       # one ring slot: the staging tile has its own memory
+    (24, 1, 70, 256, 256),       # one ring slot: the tile is turned around in two parts
+    (64, 1, 333, 384, 256),      # the same with all four column groups, two at a time
     (32, 2, 333, 512, 512),      # two slice groups per block
     (32, 5, 33, 128, 256),       # a single K chunk
     (40, 2, 500, 384, 256),      # third column group half used
@@ -114,6 +115,14 @@ def test_fragment_epilogue_edges(bm, stages, m, k, inter, offset):
     out = buf[offset:].view(m, k)
     check_close(run_capi(case, bm, 64, 4, stages, out=out), orc.run_oracle(case, bm), tag=f"bm={bm} st={stages} off={offset}")
     assert not buf[:offset].any()
+
+
+@pytest.mark.parametrize("bm,k,m", [(32, 156928, 40), (64, 79232, 70)])
+def test_fragment_epilogue_at_the_largest_hidden_size(bm, k, m):
+    """The largest K that fits one ring slot beside the scales (blocks of 64: with two epilogue warpgroups, one CTA per
+    SM); one full block and one ragged one.  Bounds as above."""
+    case = orc.make_case(1, k, 256, m, 1, seed=bm)
+    check_close(run_capi(case, bm, 64, 4, 5), orc.run_oracle(case, bm), tag=f"bm={bm} k={k}")
 
 
 def test_skewed_routing_with_empty_experts():

@@ -133,6 +133,18 @@ def test_plan_fits_shared_memory_for_every_knob():
         capi.set_ksplit(9)
 
 
+@pytest.mark.parametrize("block_m,block_n,largest", [(16, 32, 328448), (16, 64, 280576), (32, 32, 174336), (24, 64, 156928),
+                                                     (32, 64, 156928), (64, 32, 86784), (40, 64, 79232), (64, 64, 79232),
+                                                     (128, 32, 31488), (128, 64, 26752)])
+def test_largest_hidden_size_that_fits_a_ring_of_one_slot(block_m, block_n, largest):
+    """What a block needs beside its one ring slot grows with K (token and block scales): the hidden sizes accepted per
+    tile.  The staging tile of the fragment epilogue lies inside the slot and must not shorten them."""
+    from alpha_moe_b200 import capi
+    assert capi.plan(largest, block_m, 5, block_n)[0] == 1
+    with pytest.raises(capi.AlphaMoeError, match="does not fit"):
+        capi.plan(largest + 128, block_m, 5, block_n)
+
+
 def test_out_alignment_is_checked_per_kernel_before_anything_is_launched():
     """block_m > 64 accumulates with 16-byte vector reductions: an `out` that is only 4-byte aligned must be
     rejected with an argument error (it would fault on the device); block_m <= 64 accepts it.  The call with
