@@ -209,11 +209,12 @@ int launch_variant(const MapSet& maps, const amoe::MoeParams& p, int grid, int s
     return launch_dependent(kern, grid, threads, smem_bytes, p.ksplit, stream, maps, p);
 }
 
-// A shape with the fragment epilogue: a ring of one slot takes its general form (see the kernel).
+// A shape with the fragment epilogue: a ring of one slot and an `out` that is only 4-byte aligned take its general form
+// (see the kernel).
 template <int BMP, int EW, bool PEERS>
 int launch_frag(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
-    return p.stages == 1 ? launch_variant<BMP, 2, EW, PEERS, true>(maps, p, grid, smem_bytes, dev, stream)
-                         : launch_variant<BMP, 2, EW, PEERS, false>(maps, p, grid, smem_bytes, dev, stream);
+    return p.stages == 1 || !p.out_vec16 ? launch_variant<BMP, 2, EW, PEERS, true>(maps, p, grid, smem_bytes, dev, stream)
+                                          : launch_variant<BMP, 2, EW, PEERS, false>(maps, p, grid, smem_bytes, dev, stream);
 }
 
 template <int SPC>

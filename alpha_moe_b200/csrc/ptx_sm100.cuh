@@ -415,13 +415,12 @@ __device__ __forceinline__ void red_add_v4_bf16x2_raw_if(__nv_bfloat16* addr, co
         "@p red.global.add.noftz.v4.bf16x2 [%0], {%1, %2, %3, %4};\n\t}"
         ::"l"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(static_cast<uint32_t>(pred)));
 }
-// The same for an address that is only 4-byte aligned.
-__device__ __forceinline__ void red_add_4x_bf16x2_raw_if(__nv_bfloat16* addr, const uint4& w, bool pred) {
+// One packed pair, issued only where `pred` holds.
+__device__ __forceinline__ void red_add_bf16x2_raw_if(__nv_bfloat16* addr, uint32_t w, bool pred) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t"
-        "@p red.global.add.noftz.bf16x2 [%0], %1;\n\t@p red.global.add.noftz.bf16x2 [%0 + 4], %2;\n\t"
-        "@p red.global.add.noftz.bf16x2 [%0 + 8], %3;\n\t@p red.global.add.noftz.bf16x2 [%0 + 12], %4;\n\t}"
-        ::"l"(addr), "r"(w.x), "r"(w.y), "r"(w.z), "r"(w.w), "r"(static_cast<uint32_t>(pred)));
+        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t"
+        "@p red.global.add.noftz.bf16x2 [%0], %1;\n\t}"
+        ::"l"(addr), "r"(w), "r"(static_cast<uint32_t>(pred)));
 }
 // Register re-balancing between warpgroups (all four warps of a warpgroup must execute it).
 template <int N>
