@@ -333,7 +333,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const uint32_t aph = (it >> 1) & 1;
             const float sx = xs[kc * kTmRows + t];
             const float fg = sx * swg[sl * KC + kc], fu = sx * swu[sl * KC + kc];
-            if (!mbar_wait(&acc_full[b], aph, abort_flag, p.status, 40, it)) { ok = false; break; }
+            if (!mbar_wait(&acc_full[b], aph, abort_flag, p.status, 40, it)) ok = false;
             tc_fence_after();
             if (warp_valid) {
                 const uint32_t tb = tlane + b * 256 + hh * 128;
@@ -359,7 +359,8 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                 }
             }
             tc_fence_before();
-            __syncwarp();
+            ok = __all_sync(0xFFFFFFFFu, ok);      // (see fused_moe_kernel.cuh: the warp leaves a loop as a whole)
+            if (!ok) break;
             if (lane == 0) mbar_arrive_relaxed(&acc_empty[b]);
         }
             if (ok) {
@@ -380,7 +381,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                 amaxx[hh * kTmRows + t] = __float_as_uint(amax);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&xchg[0]);
-                if (!mbar_wait(&xchg[0], xph, abort_flag, p.status, 42, sl)) ok = false;
+                ok = mbar_wait_warp(&xchg[0], xph, abort_flag, p.status, 42, sl);
                 xph ^= 1;
                 amax = fmaxf(amax, __uint_as_float(amaxx[(hh ^ 1) * kTmRows + t]));
                 const float s_h = fmaxf(amax, 1e-10f) * (1.0f / 448.0f);
@@ -455,7 +456,8 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const int b = it & 1;
             const uint32_t aph = (it >> 1) & 1;
             if ((jt & 1) != hh) continue;
-            if (!mbar_wait(&acc_full[b], aph, abort_flag, p.status, 41, it)) { ok = false; break; }
+            ok = mbar_wait_warp(&acc_full[b], aph, abort_flag, p.status, 41, it);
+            if (!ok) break;
             tc_fence_after();
 #pragma unroll
             for (int part = 0; part < PARTS; ++part) {
