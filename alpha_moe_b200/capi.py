@@ -144,7 +144,8 @@ def align_workspace_bytes(numel: int, num_experts: int) -> int:
 
 def quant_and_align(x_bf16, x_fp8, x_scale, M, K, zero_src, topk_ids, top_k, num_experts, block_m, sorted_token_ids,
                     expert_ids, num_tokens_post_padded, workspace=None, stream=0) -> None:
-    """Quantisation of the activations and the block schedule, as one launch when M * top_k <= 2048."""
+    """Quantisation of the activations and the block schedule, as one launch for decode-size
+    batches (M * top_k <= 1024, and up to 2048 while schedule and activations are small)."""
     _check(lib.alpha_moe_b200_quant_and_align(x_bf16, x_fp8, x_scale, M, K, int(zero_src), topk_ids, top_k, num_experts,
                                               block_m, sorted_token_ids, expert_ids, num_tokens_post_padded, workspace,
                                               stream))

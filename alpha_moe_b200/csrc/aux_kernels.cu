@@ -40,8 +40,8 @@ using amoe_capi::fail;
 //   phase C  stable scatter: warps walk their 128 assignments in order, ranking equal experts inside a warp round
 //            with match.any
 // One launch runs all three phases with a grid-wide barrier after phase A (a cooperative launch, used whenever all
-// chunks fit on the GPU at once); otherwise phase A and phases B + C are two launches of the same kernel.  Up
-// to kSingleMax assignments are the work of one CTA of an ordinary launch (align_single_body).
+// chunks fit on the GPU at once); otherwise phase A and phases B + C are two launches of the same kernel.  Small
+// schedules are the work of one CTA of an ordinary launch (align_single_body, single_cta_schedule).
 // Programmatic dependent launch: the kernel behind this one in the stream (the fused operator, which is launched with
 // the matching attribute and waits for this kernel's completion before it reads anything) may be scheduled from here on.
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
@@ -176,7 +176,7 @@ moe_align_chunks_kernel(const int32_t* ids, int numel, int E, int block, int32_t
 
 // Everything in one CTA for up to kSingleMax assignments (227 tokens at top_k = 9).  Nothing here is more than a few
 // kilobytes; what counts is the number of dependent steps, so every load of an id is issued first, the default fills are
-// 16-byte stores, and there are three barriers.  Warp w owns 32 * rounds consecutive assignments; cnt[w][e] counts its
+// 16-byte stores, and there are four barriers.  Warp w owns 32 * rounds consecutive assignments; cnt[w][e] counts its
 // assignments of expert e, then (after thread t has turned the columns of its experts into exclusive sums over the
 // warps) it is the number of earlier ones, and start[e] the expert's first slot.
 // The line to the kernel with one CTA per 1024 assignments and a grid-wide barrier, in the call that also quantises (one
@@ -184,10 +184,26 @@ moe_align_chunks_kernel(const int32_t* ids, int numel, int E, int block, int32_t
 // assignments, with 16 rounds) 19.5 against 12.8 - match.any takes longer than a grid-wide barrier from about there on.
 // Few rounds also keep the code short, and at these sizes it is fetched cold: 1 token 4.1 -> 3.6 us, 24 tokens 6.4 -> 4.6,
 // 96 tokens at 512 experts 7.2 -> 6.2 (before: 256 threads, a serial walk of four rounds per warp).
+// Above 1024 assignments the default fills count too: they are all this one CTA's stores, where the other kernel has two
+// CTAs.  2048 assignments (four rounds) and 132096 slots 16.8 us against 15.2, 67072 slots 11.9 against 11.5, 66560 slots
+// 12.6 against 12.9; 1100 assignments (three rounds) and 131148 slots 14.8 against 15.2, 65612 slots 10.7 against 12.9:
+// the line is at rounds x slots.
 constexpr int kSingleThreads = 512;
 constexpr int kSingleWarps = kSingleThreads / 32;
 constexpr int kSingleRounds = 4;
 constexpr int kSingleMax = kSingleThreads * kSingleRounds;
+
+constexpr long long kSingleRoundSlots = 400000;
+
+inline bool single_cta_schedule(long long numel, long long sorted_len) {
+    const long long rounds = (numel + kSingleThreads - 1) / kSingleThreads;
+    return numel <= kChunk || (numel <= kSingleMax && rounds * sorted_len <= kSingleRoundSlots);
+}
+
+// Above 1024 assignments the quantiser's work counts as well: in one launch with the schedule it has two CTAs of 16 warps
+// per SM, on its own up to 64 warps.  Groups of 128 values (with the source cleared), two launches and one: 57400 9.3 and
+// 7.5 us, 78400 9.6 and 9.7, 89600 10.2 and 10.7, 114688 11.8 and 13.3, 131200 12.8 and 14.0.
+constexpr long long kSingleGroups = 80000;
 
 struct SingleSmem {
     uint32_t cnt[kSingleWarps * kMaxExperts / 2];      // two 16-bit counters a word: kSingleMax fits 16 bits
@@ -455,9 +471,9 @@ int64_t alpha_moe_b200_align_workspace_bytes(int numel, int num_experts) {
     return chunks <= 1 ? 0 : chunks * num_experts * static_cast<int64_t>(sizeof(int));
 }
 
-int alpha_moe_b200_moe_align_block_size(const int32_t* topk_ids, int numel, int num_experts, int block_m,
-                                        int32_t* sorted_token_ids, int32_t* expert_ids,
-                                        int32_t* num_tokens_post_padded, void* workspace, void* stream) {
+// single_cta: whether a schedule that fits one CTA may go to the kernel of one CTA.
+static int launch_schedule(const int32_t* topk_ids, int numel, int num_experts, int block_m, int32_t* sorted_token_ids,
+                           int32_t* expert_ids, int32_t* num_tokens_post_padded, void* workspace, void* stream, bool single_cta) {
     using namespace amoe_aux;
     if (!topk_ids || !sorted_token_ids || !expert_ids || !num_tokens_post_padded)
         return fail(ALPHA_MOE_E_ARG, "null pointer argument");
@@ -471,7 +487,7 @@ int alpha_moe_b200_moe_align_block_size(const int32_t* topk_ids, int numel, int 
     const int chunks = (numel + kChunk - 1) / kChunk;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     if (chunks > 1 && !workspace) return fail(ALPHA_MOE_E_ARG, "workspace is required for more than %d assignments", kChunk);
-    if (numel <= kSingleMax) {
+    if (single_cta && single_cta_schedule(numel, sorted_len)) {
         moe_align_single_kernel<<<1, kSingleThreads, 0, st>>>(topk_ids, numel, num_experts, block_m, sorted_token_ids,
                                                             static_cast<int>(sorted_len), expert_ids, n_blocks_max,
                                                             num_tokens_post_padded);
@@ -513,6 +529,13 @@ int alpha_moe_b200_moe_align_block_size(const int32_t* topk_ids, int numel, int 
                                                              num_tokens_post_padded, kPhaseBC);
     AUX_TRY(cudaGetLastError());
     return ALPHA_MOE_OK;
+}
+
+int alpha_moe_b200_moe_align_block_size(const int32_t* topk_ids, int numel, int num_experts, int block_m,
+                                        int32_t* sorted_token_ids, int32_t* expert_ids,
+                                        int32_t* num_tokens_post_padded, void* workspace, void* stream) {
+    return launch_schedule(topk_ids, numel, num_experts, block_m, sorted_token_ids, expert_ids, num_tokens_post_padded,
+                           workspace, stream, true);
 }
 
 int alpha_moe_b200_moe_align_block_size_noalloc(const int32_t* topk_ids, int numel, int num_experts, int block_m,
@@ -579,19 +602,21 @@ int alpha_moe_b200_quant_and_align(void* x_bf16, void* x_fp8, float* x_scale, in
     if (num_experts <= 0 || num_experts > kMaxExperts)
         return fail(ALPHA_MOE_E_ARG, "num_experts must be in 1..%d (got %d)", kMaxExperts, num_experts);
     if (block_m <= 0) return fail(ALPHA_MOE_E_ARG, "block_m must be positive (got %d)", block_m);
-    if (numel > kSingleMax) {
-        // Two launches (the schedule needs several CTAs and a grid-wide barrier) that do not depend on each other: the
-        // schedule runs on a side stream forked from the caller's and joined back into it, beside the quantiser.  It
-        // is launched first so that its few CTAs have their places before the quantiser's grid fills every SM.
+    const long long sorted_len = numel + static_cast<long long>(num_experts) * (block_m - 1);
+    const long long n_groups = static_cast<long long>(M) * (K / 128);
+    if (!single_cta_schedule(numel, sorted_len) || (numel > kChunk && n_groups > kSingleGroups)) {
+        // Two launches that do not depend on each other: the schedule (several CTAs and a grid-wide barrier) runs on a side
+        // stream forked from the caller's and joined back into it, beside the quantiser.  It is launched first so that its
+        // few CTAs have their places before the quantiser's grid fills every SM.  (The one-CTA schedule is no gain there:
+        // 2048 assignments beside 114688 groups 12.3 us against 11.8.)
         cudaStream_t user = static_cast<cudaStream_t>(stream);
         int dev = 0;
         AUX_TRY(cudaGetDevice(&dev));
         SideStream* side = side_stream(dev);
         const bool forked = side && cudaEventRecord(side->fork, user) == cudaSuccess &&
                             cudaStreamWaitEvent(side->stream, side->fork, 0) == cudaSuccess;
-        const int rc_align = alpha_moe_b200_moe_align_block_size(topk_ids, static_cast<int>(numel), num_experts, block_m,
-                                                                 sorted_token_ids, expert_ids, num_tokens_post_padded,
-                                                                 workspace, forked ? side->stream : user);
+        const int rc_align = launch_schedule(topk_ids, static_cast<int>(numel), num_experts, block_m, sorted_token_ids,
+                                             expert_ids, num_tokens_post_padded, workspace, forked ? side->stream : user, false);
         const int rc_quant = rc_align ? rc_align
                                       : alpha_moe_b200_per_token_group_quant_fp8(x_bf16, x_fp8, x_scale, M, K, zero_src, stream);
         if (forked) {            // joined whatever happened above: the side stream never stays attached to a capture
@@ -601,11 +626,9 @@ int alpha_moe_b200_quant_and_align(void* x_bf16, void* x_fp8, float* x_scale, in
         return rc_quant;
     }
     if (numel > kChunk && !workspace) return fail(ALPHA_MOE_E_ARG, "workspace is required for more than %d assignments", kChunk);
-    const long long sorted_len = numel + static_cast<long long>(num_experts) * (block_m - 1);
     if (sorted_len > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "schedule too long for int32 indices");
     const int n_blocks_max = static_cast<int>((sorted_len + block_m - 1) / block_m);
-    const long long n_groups = static_cast<long long>(M) * (K / 128);
-    // a warp takes four groups per step; beyond 16 steps' worth of warps per SM the rest is covered by the stride
+    // a warp takes four groups per step; beyond four CTAs per SM the rest is covered by the stride
     int dev = 0, sms = 0;
     AUX_TRY(cudaGetDevice(&dev));
     AUX_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -51,7 +51,8 @@ sglang_per_token_group_quant_fp8 = per_token_group_quant_fp8   # the name used a
 def quant_and_align(x: torch.Tensor, topk_ids: torch.Tensor, block_size: int, num_experts: int,
                     zero_input: bool = False):
     """Both steps above in one call: (x_q, x_scale, sorted_token_ids, expert_ids, num_tokens_post_padded), the same
-    bits as per_token_group_quant_fp8 + moe_align_block_size.  One kernel launch when M * top_k <= 2048."""
+    bits as per_token_group_quant_fp8 + moe_align_block_size.  One kernel launch when M * top_k <= 1024, and up
+    to 2048 while schedule and activations are small."""
     if not x.is_cuda or x.dtype != torch.bfloat16 or not x.is_contiguous() or x.dim() != 2:
         raise RuntimeError("x must be a contiguous 2-D bfloat16 CUDA tensor")
     if not topk_ids.is_cuda or topk_ids.dim() != 2 or topk_ids.shape[0] != x.shape[0]:

@@ -26,9 +26,10 @@ def test_moe_align_block_size_matches_oracle_exactly(m, e, k, block):
 @pytest.mark.parametrize("numel", [1, 31, 32, 33, 512, 513, 1024, 1025, 1537, 2047, 2048, 2049])
 @pytest.mark.parametrize("e,block", [(1, 8), (257, 16), (1023, 8), (1024, 128)])
 def test_schedule_at_the_edges_of_the_single_cta_kernel(numel, e, block):
-    """One CTA builds the schedule of up to 2048 assignments (16 warps of up to four rounds of 32), more take the
-    multi-CTA kernel: exact on both sides of every edge, with one expert and with the most there can be, for random
-    ids and for all assignments going to the last expert."""
+    """One CTA builds the schedule of up to 2048 assignments (16 warps of up to four rounds of 32); more, and more than
+    1024 with very many slots to fill (1024 experts, blocks of 128), take the multi-CTA kernel: exact on both sides of
+    every edge, with one expert and with the most there can be, for random ids and for all assignments going to the last
+    expert."""
     from alpha_moe_b200.prologue import moe_align_block_size
     g = torch.Generator().manual_seed(numel + e)
     for ids in (torch.randint(0, e, (numel, 1), generator=g, dtype=torch.int32),
@@ -97,10 +98,12 @@ def test_group_quant_matches_oracle_bit_for_bit(m, k):
 
 @pytest.mark.parametrize("m,e,k,hidden,block", [(1, 257, 9, 7168, 16), (7, 8, 2, 128, 8), (64, 512, 10, 2048, 16),
                                                 (113, 257, 9, 7168, 32), (114, 257, 9, 7168, 16), (500, 37, 9, 1024, 64),
-                                                (227, 257, 9, 7168, 16), (228, 257, 9, 1024, 16)])
+                                                (227, 257, 9, 7168, 16), (228, 257, 9, 1024, 16),
+                                                (1100, 64, 1, 9216, 64), (1100, 64, 1, 9344, 64), (2048, 1024, 1, 128, 128)])
 def test_quant_and_align_in_one_call_matches_oracle_bit_for_bit(m, e, k, hidden, block):
-    """Quantisation and schedule as one launch (M * top_k <= 2048) or as the two separate
-    launches (the rest), against the CPU restatement of each; with and without clearing the source."""
+    """Quantisation and schedule as one launch (M * top_k <= 1024, or up to 2048 with few slots and groups) or as the two
+    separate launches (the rest), on both sides of each line, against the CPU restatement of each; with and without
+    clearing the source."""
     from alpha_moe_b200.prologue import quant_and_align
     g = torch.Generator().manual_seed(3 * m + e)
     x = (torch.randn(m, hidden, generator=g) * torch.rand(m, 1, generator=g) * 3).to(torch.bfloat16)

@@ -247,7 +247,7 @@ def test_tensor_parallel_entry_points_reject_bad_arguments_before_any_launch():
 
 def test_quant_and_align_entry_rejects_bad_arguments_before_any_launch():
     """alpha_moe_b200_quant_and_align (both steps in front of the operator in one call): argument errors come back as
-    error codes from both of its forms - one launch (M * top_k <= 1024) and two launches - without touching a GPU."""
+    error codes from both of its forms - one launch (small batches) and two launches - without touching a GPU."""
     from alpha_moe_b200 import capi
     p = 0x10000
     base = dict(x_bf16=p, x_fp8=p, x_scale=p, M=4, K=512, zero_src=1, topk_ids=p, top_k=2, num_experts=8, block_m=16,
