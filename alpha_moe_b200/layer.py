@@ -12,6 +12,12 @@ import torch
 from . import capi
 from .utils import get_best_config
 
+try:        # the raw handle without a Stream object around it (one microsecond of an eager call's host time)
+    from torch._C import _cuda_getCurrentRawStream as _current_stream
+except ImportError:
+    def _current_stream(device_index: int) -> int:
+        return torch.cuda.current_stream(device_index).cuda_stream
+
 
 def _up(n: int) -> int:
     return (n + 255) & ~255
@@ -107,5 +113,5 @@ def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: 
                            w2.data_ptr(), w2_scale.data_ptr(), ids.data_ptr(), wts.data_ptr(), top_k, m, k, n, e,
                            base + sorted_ids, base + expert_ids, base + num_post_pad, base + ws if ws_bytes else 0,
                            block_m, bn, wn, stages, float(routed_scaling_factor or 1.0),
-                           torch._C._cuda_getCurrentRawStream(dev.index))
+                           _current_stream(dev.index))
     return hidden_states
