@@ -40,6 +40,31 @@ def test_schedule_at_the_edges_of_the_single_cta_kernel(numel, e, block):
             assert torch.equal(a.cpu(), b), name
 
 
+@pytest.mark.parametrize("numel", [1, 33, 700, 1024, 1500, 2048])
+@pytest.mark.parametrize("e", [8, 257])
+def test_small_schedules_ignore_ids_out_of_range(numel, e):
+    """The one-CTA schedule counts and scatters only ids in [0, E): -1, E and large ids take no slot, wherever they stand
+    in a warp, and with nothing else there is no block at all."""
+    from alpha_moe_b200.prologue import moe_align_block_size
+    g = torch.Generator().manual_seed(numel + e)
+    ids = torch.randint(0, e, (numel, 1), generator=g, dtype=torch.int32)
+    bad = torch.tensor([-1, e, 1 << 30, -(1 << 31)], dtype=torch.int32)
+    hit = torch.rand(numel, generator=g) < 0.3
+    ids[hit, 0] = bad[torch.randint(0, 4, (int(hit.sum()),), generator=g)]
+    sid, eid, npp = [t.cpu() for t in moe_align_block_size(ids.cuda(), 16, e)]
+    want, blocks = [], []
+    for x in range(e):
+        mine = [i for i in range(numel) if int(ids[i]) == x]
+        pad = -len(mine) % 16
+        want += mine + [numel] * pad
+        blocks += [x] * ((len(mine) + pad) // 16)
+    assert int(npp) == len(want) and sid[:len(want)].tolist() == want and eid[:len(blocks)].tolist() == blocks
+    assert (sid[len(want):] == numel).all()
+    none = bad[torch.randint(0, 4, (numel, 1), generator=g)]
+    sid, eid, npp = moe_align_block_size(none.cuda(), 16, e)
+    assert int(npp) == 0 and bool((sid == numel).all())
+
+
 def test_moe_align_more_chunks_than_fit_on_the_gpu_and_many_experts():
     """About a million assignments are more 1024-assignment chunks than can be resident at once, so the schedule is
     built by two launches instead of one cooperative launch; 1000 experts exercises several experts per thread in

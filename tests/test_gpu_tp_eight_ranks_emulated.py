@@ -32,19 +32,27 @@ def _flags(preset: int):
     return flags
 
 
-def test_operator_adds_into_all_eight_out_buffers():
+@pytest.mark.parametrize("inter,m,shapes", [
+    (1024, 24, ((16, 32, 8, 3), (64, 32, 8, 2))),                        # one slice per CTA
+    (2048, 90, ((32, 64, 4, 3), (32, 64, 4, 1), (64, 64, 4, 3), (64, 64, 4, 1))),      # two: the fragment epilogue
+])
+@pytest.mark.parametrize("offset", [0, 2])
+def test_operator_adds_into_all_eight_out_buffers(inter, m, shapes, offset):
+    """Every rank's partial result is added into all eight buffers.  offset: one rank's buffer starts that many values
+    later, so that it is only 4-byte aligned - then no buffer may be reduced into in 16-byte pieces."""
     from alpha_moe_b200 import capi
     from alpha_moe_b200.tp import shard_weights
-    e, k, inter, m, top_k = 8, 1024, 1024, 24, 3
+    e, k, top_k = 8, 1024, 3
     g = torch.Generator().manual_seed(808)
     weights = orc.make_weights(e, k, inter, g)
     case = orc.make_case(e, k, inter, m, top_k, seed=809, scaling=1.5, weights=weights)
     full = [t.cuda() for t in weights]
-    for bm, bn, wn, st in ((16, 32, 8, 3), (64, 32, 8, 2)):
+    for bm, bn, wn, st in shapes:
         sid, eid, npp = [t.cuda() for t in case.schedule(bm)]
         x, xs, wts = case.x.cuda(), case.x_scale.cuda(), case.topk_weights.cuda()
-        outs = [torch.zeros(m, k, dtype=torch.bfloat16, device="cuda") for _ in range(WORLD)]
-        ptrs = [o.data_ptr() for o in outs]
+        bufs = [torch.zeros(m * k + 2, dtype=torch.bfloat16, device="cuda") for _ in range(WORLD)]
+        starts = [offset if r == 5 else 0 for r in range(WORLD)]
+        ptrs = [b.data_ptr() + 2 * o for b, o in zip(bufs, starts)]
         keep = []
         for rank in range(WORLD):
             w, w_scale, w2, w2_scale = shard_weights(*full, rank, WORLD)
@@ -56,8 +64,9 @@ def test_operator_adds_into_all_eight_out_buffers():
         torch.cuda.synchronize()
         assert capi.read_status(reset=True)[0] == 0
         ref = orc.run_oracle(case, bm)
-        for rank, o in enumerate(outs):
-            assert orc.rel_l2(o.cpu(), ref) <= 2e-2, (bm, rank)
+        for rank, (b, o) in enumerate(zip(bufs, starts)):
+            assert orc.rel_l2(b[o:o + m * k].view(m, k).cpu(), ref) <= 2e-2, (bm, st, rank)
+            assert not b[:o].any() and not b[o + m * k:].any()
 
 
 @pytest.mark.parametrize("n", [8 * 7, 7168, 64 * 7168 + 8])
