@@ -65,8 +65,9 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                                              const __grid_constant__ CUtensorMap tm_w2, const MoeParams p) {
     constexpr int EPI_THREADS = 256;
     // control warpgroup: weight TMA, gather, UMMA (even chunks), UMMA (odd chunks); then four more gather warps.
-    // One warp issues a 16-byte cp.async of 32 lanes only about every 100 cycles, whatever the addresses, and a
-    // 128-row x 128-byte token tile takes 32 of them: five warps bring a tile in about as long as its UMMAs run.
+    // A 128-row x 128-byte token tile is 32 cp.async of 32 lanes x 16 bytes.  A warp issues one in 7-15 cycles, but they are
+    // in flight for several hundred (five warps x 16 of them are done in about 520): five warps bring a tile in about as
+    // long as its UMMAs run.
     constexpr int W_TMA = 8, W_G0 = 9, W_MMA0 = 10, W_G1 = 12;
     constexpr int GATHER_THREADS = kTmGatherWarps * 32;
     constexpr uint32_t TMEM_COLS = 512;
