@@ -56,6 +56,48 @@ __host__ __device__ inline SmemPlanTm smem_plan_tm(int s, int kc, int spc) {
     return p;
 }
 
+// Token scales of one token into shared memory, xs[c * PITCH] for the K chunks of units first, first + step, ... (a unit is
+// four chunks where the rows can be read as float4, else one).  All loads of a batch are in flight before the first store:
+// this stands in front of the first promotion, and a load that waits for the one before costs a memory latency each.  With the
+// sorted ids requested at kernel entry, calls in a row, DeepSeek-V3 TP8 shard, M = 4096 542 -> 535 us, M = 8192 (Zipf) 897 ->
+// 887, Qwen3-Next shard M = 4096 235 -> 233.
+template <int PITCH, int BATCH>
+__device__ __forceinline__ void stage_token_scales(float* xs, const float* row, bool live, int first, int step, int units,
+                                                   bool vec4) {
+    if (vec4) {
+        for (int u0 = first; u0 < units; u0 += BATCH * step) {
+            float4 v[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int u = u0 + i * step;
+                v[i] = live && u < units ? __ldg(reinterpret_cast<const float4*>(row) + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int u = u0 + i * step;
+                if (u < units) {
+                    xs[(4 * u) * PITCH] = v[i].x;
+                    xs[(4 * u + 1) * PITCH] = v[i].y;
+                    xs[(4 * u + 2) * PITCH] = v[i].z;
+                    xs[(4 * u + 3) * PITCH] = v[i].w;
+                }
+            }
+        }
+    } else {
+        for (int u0 = first; u0 < units; u0 += BATCH * step) {
+            float v[BATCH];
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i) {
+                const int u = u0 + i * step;
+                v[i] = live && u < units ? __ldg(row + u) : 0.f;
+            }
+#pragma unroll
+            for (int i = 0; i < BATCH; ++i)
+                if (u0 + i * step < units) xs[(u0 + i * step) * PITCH] = v[i];
+        }
+    }
+}
+
 constexpr int kTmThreads = 512;     // 2 epilogue warpgroups + control warpgroup + gather warpgroup
 constexpr int kTmGatherWarps = 5;   // one warp of the control warpgroup + the gather warpgroup
 
@@ -78,17 +120,35 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     const int slice0 = (blockIdx.x - mblock * ngroups) * SPC;
     griddep_wait();      // the schedule, the activations and the cleared `out` may come from the kernel just before
     griddep_launch_dependents();   // a kernel behind this launch may be scheduled; it waits for our completion
-    const int npad = min(p.num_tokens_post_padded[0], p.sorted_num);
-    if (mblock * p.block_m >= npad) return;
-    const int expert = p.expert_ids[mblock];
-    if (expert < 0 || expert >= p.E) return;
+    // What the rest of the prologue depends on is requested together, before the set-up: the schedule's length, this block's
+    // expert and the sorted ids this thread will need (a gather thread those of its rows, an epilogue thread its token's).
+    constexpr int GROUPS = kTmRows / 4, MAXG = (GROUPS + kTmGatherWarps - 1) / kTmGatherWarps;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int gather_warp = warp == W_G0 ? 0 : warp - W_G1 + 1;      // of the gather role only
+    int pid_pre[MAXG];
+    int expert;
+    {
+        const int npad_raw = ld_global_nc_s32(p.num_tokens_post_padded);
+        expert = ld_global_nc_s32(p.expert_ids + mblock);
+        const bool gather_role = warp == W_G0 || warp >= W_G1;
+#pragma unroll
+        for (int i = 0; i < MAXG; ++i) {
+            const int grp = gather_warp + kTmGatherWarps * i;
+            const int row = gather_role ? 4 * grp + (lane >> 3) : static_cast<int>(threadIdx.x & (kTmRows - 1));
+            const int idx = mblock * p.block_m + row;
+            pid_pre[i] = -1;
+            if ((gather_role || (i == 0 && warp < W_TMA)) && row < p.block_m && idx < p.sorted_num)
+                pid_pre[i] = ld_global_nc_s32(p.sorted_token_ids + idx);
+        }
+        if (mblock * p.block_m >= min(npad_raw, p.sorted_num)) return;
+        if (expert < 0 || expert >= p.E) return;
+    }
 
     const int KC = p.K >> 7;
     const int UPI = SPC * KC;
     const int ND = SPC == 1 ? (KC + 1) >> 1 : KC;
     const int NIT = UPI + ND;
     const int S = p.stages;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     // The operand tiles need 1024-byte alignment (128-byte swizzle atoms).  The dynamic shared memory
     // window is declared with that alignment; should a toolchain ever place it differently, the CTA
@@ -231,9 +291,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         // ------------------------------------------------------------------ token-row gather (5 warps)
         // Row group j (4 token rows x 128 B, one cp.async of the warp) belongs to gather warp j % 5: 7 groups for
         // the first two warps, 6 for the others.  Lane l copies 16-byte piece l & 7 of row 4j + (l >> 3).
-        constexpr int GROUPS = kTmRows / 4;
-        constexpr int MAXG = (GROUPS + kTmGatherWarps - 1) / kTmGatherWarps;
-        const int gw = warp == W_G0 ? 0 : warp - W_G1 + 1;
+        const int gw = gather_warp;
         const int ch = lane & 7;
         uint32_t src16[MAXG];
         uint32_t dst[MAXG];
@@ -241,16 +299,13 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         for (int i = 0; i < MAXG; ++i) {
             const int grp = gw + kTmGatherWarps * i;
             const int row = 4 * grp + (lane >> 3);
-            const int idx = mblock * p.block_m + row;
+            const int pid = pid_pre[i];            // requested at kernel entry; -1 for rows past the block
             src16[i] = 0xFFFFFFFFu;
             dst[i] = 0xFFFFFFFFu;                  // no such group for this warp
             if (grp < GROUPS) {
                 dst[i] = row * 128 + ((ch ^ (row & 7)) << 4);
-                if (row < p.block_m && idx < p.sorted_num) {
-                    const int pid = p.sorted_token_ids[idx];
-                    if (pid >= 0 && pid < p.M * p.top_k)
-                        src16[i] = static_cast<uint32_t>((static_cast<size_t>(pid / p.top_k) * p.K) >> 4);
-                }
+                if (pid >= 0 && pid < p.M * p.top_k)
+                    src16[i] = static_cast<uint32_t>((static_cast<size_t>(pid / p.top_k) * p.K) >> 4);
             }
         }
         int s = 0;
@@ -284,13 +339,10 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         int row = p.M;
         float tw = 0.f;
         {
-            const int idx = mblock * p.block_m + t;
-            if (t < p.block_m && idx < p.sorted_num) {
-                const int pid = p.sorted_token_ids[idx];
-                if (pid >= 0 && pid < p.M * p.top_k) {
-                    row = pid / p.top_k;             // reference :757
-                    tw = p.topk_weights[pid];        // reference :761
-                }
+            const int pid = pid_pre[0];
+            if (pid >= 0 && pid < p.M * p.top_k) {
+                row = pid / p.top_k;             // reference :757
+                tw = p.topk_weights[pid];        // reference :761
             }
         }
         const bool valid = row < p.M;
@@ -306,14 +358,11 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                 sw2[i] = p.w2_scale[(static_cast<size_t>(expert) * KC + c) * isl + slice0 + sl];
             }
         }
-        named_bar_sync(1, EPI_THREADS);
-
         // Token scales go to shared memory once (each warpgroup fetches one half of the K chunks of its tokens): the
         // chunk loop then holds no global load, whose latency a releasing hand-off would have to wait out.
         {
             const float* xs_row = p.x_scale + static_cast<size_t>(valid ? row : 0) * KC;
-            const int c_begin = hh * (KC >> 1), c_end = hh == 0 ? (KC >> 1) : KC;
-            for (int c = c_begin; c < c_end; ++c) xs[c * kTmRows + t] = valid ? xs_row[c] : 0.f;
+            stage_token_scales<kTmRows, 8>(xs + t, xs_row, valid, hh, 2, p.xs_vec4 ? KC >> 2 : KC, p.xs_vec4);
         }
         named_bar_sync(1, EPI_THREADS);
 

@@ -709,6 +709,7 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     p.out_vec16 = 1;
     for (int r = 0; r < tp_world; ++r)
         if (reinterpret_cast<uintptr_t>(outs[r]) & 15) p.out_vec16 = 0;
+    p.xs_vec4 = (K / 128) % 4 == 0 && (reinterpret_cast<uintptr_t>(x_scale) & 15) == 0;
     p.status = facts.status;
 
     const long long grid = nblocks * (N / 256 / spc) * ksplit;

@@ -349,3 +349,21 @@ def test_reference_timing_scripts_imbalance_model(balancedness):
     assert float((ids[:, :-1] == 0).float().mean()) > (1 - balancedness) * 0.8        # expert 0 is hot
     for bm, bn, wn, st in ((8, 64, 4, 3), (16, 32, 8, 5), (32, 64, 4, 2), (64, 64, 4, 2), (64, 32, 8, 4), (128, 64, 4, 3)):
         check_close(run_capi(case, bm, bn, wn, st), orc.run_oracle(case, bm), tag=f"mixture {balancedness} bm={bm} bn={bn}")
+
+
+@pytest.mark.parametrize("k,inter,m,bm,stages", [
+    (128, 256, 130, 128, 3),      # a single K chunk: no warpgroup has a second one to stage
+    (384, 256, 300, 96, 1),       # three chunks: the scale rows are not multiples of 16 bytes; one ring slot
+    (512, 128, 257, 128, 2),      # four chunks, one slice per CTA
+    (4608, 256, 200, 72, 4),      # 36 chunks: more 16-byte pieces than one batch of loads
+])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_token_major_scale_staging(k, inter, m, bm, stages, offset):
+    """Blocks above 64: token scales are staged as 16-byte pieces where their rows allow it (offset 0 and K/128 a multiple
+    of 4), else one by one.  Bounds as above."""
+    case = orc.make_case(3, k, inter, m, 2, seed=k + m, scaling=1.5)
+    d = to_device(case)
+    buf = torch.empty(case.x_scale.numel() + offset, device="cuda:0")
+    d["x_scale"] = buf[offset:].view(case.x_scale.shape)
+    d["x_scale"].copy_(case.x_scale)
+    check_close(run_capi(case, bm, 64, 4, stages, dcase=d), orc.run_oracle(case, bm), tag=f"k={k} bm={bm} off={offset}")
