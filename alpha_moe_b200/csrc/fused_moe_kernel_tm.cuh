@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(kTmThreads, 1)
 fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap tm_w,
                                              const __grid_constant__ CUtensorMap tm_w2, const MoeParams p) {
     constexpr int EPI_THREADS = 256;
-    // control warpgroup: weight TMA, gather, UMMA (even chunks), UMMA (odd chunks); then four more gather warps.
+    // control warpgroup: weight TMA, gather, UMMA, one warp without a role; then four more gather warps.
     // A 128-row x 128-byte token tile is 32 cp.async of 32 lanes x 16 bytes.  A warp issues one in 7-15 cycles, but they are
     // in flight for several hundred (five warps x 16 of them are done in about 520): five warps bring a tile in about as
     // long as its UMMAs run.
@@ -174,7 +174,6 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     uint64_t* xchg = h_ready + 1;
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.misc);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.misc + 4);
-    volatile int* issue_turn = reinterpret_cast<volatile int*>(smem + L.misc + 8);   // iterations whose operands have been waited for
 
     if (threadIdx.x == W_TMA * 32) {
         for (int i = 0; i < S; ++i) {
@@ -188,7 +187,6 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         mbar_init(h_ready, 1);
         mbar_init(&xchg[0], 8);
         *abort_flag = 0;
-        *issue_turn = 0;
         fence_mbar_init();
     }
     if (warp == W_MMA0) {
@@ -203,10 +201,11 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     if (warp >= W_TMA) {
     // ====================================================================== control + gather warpgroups
     setmaxnreg_dec<40>();
-    if (warp == W_MMA0 || warp == W_MMA0 + 1) {
-        // ------------------------------------------------------------------ UMMA issuers (even / odd chunks)
+    if (warp == W_MMA0 + 1) {
+        // (no role: one warp issues a chunk's four or eight UMMAs faster than they run)
+    } else if (warp == W_MMA0) {
+        // ------------------------------------------------------------------ UMMA issuer
         {
-            const int pw = warp - W_MMA0;
             constexpr uint32_t idesc256 = umma_idesc_e4m3(128, 256);
             constexpr uint32_t idesc128 = umma_idesc_e4m3(128, 128);
             const uint32_t st0 = smem_u32(smem);
@@ -216,11 +215,10 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const uint64_t x_0 = umma_desc_sw128(st0 + 2 * kTileBytes);     // gathered token rows (M operand)
             const uint64_t h0 = umma_desc_sw128(smem_u32(hq));
             const uint64_t h1 = umma_desc_sw128(smem_u32(hq + (SPC - 1) * kTmRows * 128));
-            const int step = S > 1 ? 2 : 1;      // see fused_moe_kernel.cuh: one issuer when the ring has one slot
-            int s = pw % S;
+            int s = 0;
             uint32_t ph = 0;
             bool h_waited = false;
-            for (int it = pw; it < NIT && pw < step; it += step) {
+            for (int it = 0; it < NIT; ++it) {
                 const int b = it & 1;
                 const uint32_t aph = (it >> 1) & 1;
                 const uint32_t d = tmem_base + b * 256;
@@ -230,17 +228,10 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     h_waited = true;
                 }
                 if (!mbar_wait_warp(&acc_empty[b], aph ^ 1, abort_flag, p.status, 21, it)) break;
-                // The two issuers take their turns in iteration order.  A parity wait is only meaningful while
-                // the waiter is at most one phase ahead of the barrier: waiting for fill n of a slot presumes
-                // that fill n-1 has completed.  Fill n-1 belongs to iteration it-S, which with an odd ring depth
-                // is the other issuer's; in the down phase the two warpgroups of the epilogue release the
-                // accumulator buffers independently, so without the turn one issuer could get that far ahead.
-                if (!turn_wait_warp(issue_turn, it, abort_flag, p.status, 23)) break;
                 if (!mbar_wait_warp(&full[s], ph, abort_flag, p.status, 22, it)) break;
                 tc_fence_after();
                 const uint64_t off = static_cast<uint64_t>(s * dstep);
                 if (elect_one()) {
-                    *issue_turn = it + 1;
                     fence_proxy_async_smem();  // token rows were written by cp.async, the UMMA reads them through the async proxy
                     if (up) {
                         umma_f8_chunk1(d, x_0 + off, w_0 + off, idesc256);           // D[token, 256 interleaved w rows]
@@ -253,8 +244,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     umma_commit(&empty[s]);    // the ring slot is free once these MMAs have read it
                 }
                 __syncwarp();
-                s += step;
-                while (s >= S) { s -= S; ph ^= 1; }
+                if (++s == S) { s = 0; ph ^= 1; }
             }
         }
     } else if (warp == W_TMA) {
@@ -366,18 +356,26 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         }
         named_bar_sync(1, EPI_THREADS);
 
-        // accumulators of this token: 8 groups of (8 gate, 8 up) columns = 64 intermediate columns
-        float acc[128];
+        // Accumulators of this token: 8 groups of (8 gate, 8 up) columns = 64 intermediate columns, as packed pairs.  In a row
+        // of calls this kernel runs at the power limit, where an instruction saved counts even if its unit was not busy.  Packed
+        // FMAs, the rows of the down phase's reductions in registers instead of a shuffle and a 64-bit multiplication for each,
+        // no vote per chunk and one issuing warp instead of two that took turns: DeepSeek-V3 TP8 shard, M = 4096 535 -> 514 us,
+        // M = 8192 (Zipf) 887 -> 846, unsharded M = 4096 4015 -> 3886, Qwen3-Next shard M = 4096 233 -> 220 (the rows alone
+        // are two thirds of it).  For the same reason token rows of padding stay zero: left as they are, M = 4096 is 3 % slower.
+        f32x2 acc[64];
 #pragma unroll
-        for (int j = 0; j < 128; ++j) acc[j] = 0.f;
+        for (int j = 0; j < 64; ++j) acc[j] = 0;
         float fac[SPC];                      // s_h * topk weight * scaling per slice (reference :997-1003)
 
         const uint32_t tlane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
+        // A wait that runs out does not leave the loops of the up phase: the abort flag lets every later wait return at once, and
+        // what was computed meanwhile is added nowhere (see in front of the down phase).
         bool ok = true;
         uint32_t xph = 0;
         // ---- up-projection: promote each K chunk with its scales (reference :915-933).  The chunk loop is kept
         // small and contiguous (the slice-end code follows it instead of sitting inside it).
-        for (int sl = 0, it = 0; sl < SPC && ok; ++sl) {
+        for (int sl = 0, it = 0; sl < SPC; ++sl) {
+#pragma unroll 1
         for (int kc = 0; kc < KC; ++kc, ++it) {
             const int b = it & 1;
             const uint32_t aph = (it >> 1) & 1;
@@ -385,53 +383,62 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const float fg = sx * swg[sl * KC + kc], fu = sx * swu[sl * KC + kc];
             if (!mbar_wait(&acc_full[b], aph, abort_flag, p.status, 40, it)) ok = false;
             tc_fence_after();
+            // 64 columns are requested before the first is used (every wait lengthens the chain issue -> read-back -> hand-back
+            // around the two accumulator buffers): against waits after every 32 columns, blocks of 128 at the DeepSeek-V3 TP8
+            // shard, M = 4096 460 -> 449 us, M = 8192 (Zipf) 769 -> 754 us, unsharded M = 4096 3540 -> 3212 us.  TMEM loads do
+            // not wait for UMMAs in flight: 16 columns and their FMAs take 40 cycles either way.
+            const uint32_t tb = tlane + b * 256 + hh * 128;
+            uint32_t v[4][16];
+            const f32x2 fg2 = pack_f32x2(fg, fg), fu2 = pack_f32x2(fu, fu);
+            auto request = [&](int c0) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c) tmem_ld16(tb + c0 + 16 * c, v[c]);
+                tmem_ld_wait();
+            };
+            auto promote = [&](int c0) {
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const int j = (c0 + 16 * c) / 2 + e;
+                        acc[j] = fma_f32x2(pack_u32x2(v[c][2 * e], v[c][2 * e + 1]), fg2, acc[j]);
+                        acc[j + 4] = fma_f32x2(pack_u32x2(v[c][8 + 2 * e], v[c][9 + 2 * e]), fu2, acc[j + 4]);
+                    }
+            };
             if (warp_valid) {
-                const uint32_t tb = tlane + b * 256 + hh * 128;
-                // 64 columns are requested before the first is used (every wait lengthens the chain issue -> read-back ->
-                // hand-back around the two accumulator buffers): against waits after every 32 columns, blocks of 128 at
-                // the DeepSeek-V3 TP8 shard, M = 4096 460 -> 449 us, M = 8192 (Zipf) 769 -> 754 us, unsharded M = 4096
-                // 3540 -> 3212 us.  TMEM loads do not wait for UMMAs in flight: 16 columns and their FMAs take 40 cycles
-                // either way.
-#pragma unroll
-                for (int c0 = 0; c0 < 128; c0 += 64) {
-                    uint32_t v[4][16];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) tmem_ld16(tb + c0 + 16 * c, v[c]);
-                    tmem_ld_wait();
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) {
-                            const int j = c0 + 16 * c + e;
-                            acc[j] = fmaf(__uint_as_float(v[c][e]), fg, acc[j]);
-                            acc[j + 8] = fmaf(__uint_as_float(v[c][8 + e]), fu, acc[j + 8]);
-                        }
-                }
+                request(0);
+                promote(0);
+                request(64);
+                promote(64);
             }
             tc_fence_before();
-            ok = __all_sync(0xFFFFFFFFu, ok);      // (see fused_moe_kernel.cuh: the warp leaves a loop as a whole)
-            if (!ok) break;
+            __syncwarp();
             if (lane == 0) mbar_arrive_relaxed(&acc_empty[b]);
         }
-            if (ok) {
+            {
                 // ---- end of a slice: SwiGLU, amax over the slice's 128 columns (64 here + 64 in the partner
                 //      warpgroup's thread of the same token), fp8 re-quantisation (reference :936-1005)
                 float amax = 0.f;
 #pragma unroll
                 for (int g8 = 0; g8 < 8; ++g8) {
 #pragma unroll
-                    for (int e = 0; e < 8; ++e) {
-                        const float g = bf16_round(acc[16 * g8 + e]);
-                        const float u = bf16_round(acc[16 * g8 + 8 + e]);
-                        const float h = bf16_round(__fdividef(g, 1.0f + __expf(-g)) * u);
-                        acc[16 * g8 + e] = h;
-                        amax = fmaxf(amax, fabsf(h));
+                    for (int e = 0; e < 4; ++e) {
+                        float gv[2], uv[2], h[2];
+                        unpack_f32x2(acc[8 * g8 + e], gv[0], gv[1]);
+                        unpack_f32x2(acc[8 * g8 + 4 + e], uv[0], uv[1]);
+#pragma unroll
+                        for (int i = 0; i < 2; ++i) {
+                            const float g = bf16_round(gv[i]), u = bf16_round(uv[i]);
+                            h[i] = bf16_round(__fdividef(g, 1.0f + __expf(-g)) * u);
+                            amax = fmaxf(amax, fabsf(h[i]));
+                        }
+                        acc[8 * g8 + e] = pack_f32x2(h[0], h[1]);
                     }
                 }
                 amaxx[hh * kTmRows + t] = __float_as_uint(amax);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&xchg[0]);
-                ok = mbar_wait_warp(&xchg[0], xph, abort_flag, p.status, 42, sl);
+                if (!mbar_wait(&xchg[0], xph, abort_flag, p.status, 42, sl)) ok = false;
                 xph ^= 1;
                 amax = fmaxf(amax, __uint_as_float(amaxx[(hh ^ 1) * kTmRows + t]));
                 const float s_h = fmaxf(amax, 1e-10f) * (1.0f / 448.0f);
@@ -441,11 +448,12 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     uint32_t w4[4];
 #pragma unroll
                     for (int k2 = 0; k2 < 4; ++k2) {
-                        const int base = 16 * (2 * i + (k2 >> 1)) + 4 * (k2 & 1);
+                        const int base = 8 * (2 * i + (k2 >> 1)) + 2 * (k2 & 1);
                         float qv[4];
+                        unpack_f32x2(acc[base], qv[0], qv[1]);
+                        unpack_f32x2(acc[base + 1], qv[2], qv[3]);
 #pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            qv[e] = fminf(fmaxf(__fdividef(acc[base + e], s_h), -448.0f), 448.0f);
+                        for (int e = 0; e < 4; ++e) qv[e] = fminf(fmaxf(__fdividef(qv[e], s_h), -448.0f), 448.0f);
                         const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(qv[0], qv[1]), __NV_SATFINITE, __NV_E4M3);
                         const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(qv[2], qv[3]), __NV_SATFINITE, __NV_E4M3);
                         w4[k2] = lo | (hi << 16);
@@ -455,7 +463,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                 }
                 fac[sl] = s_h * tw * p.scaling;
 #pragma unroll
-                for (int j = 0; j < 128; ++j) acc[j] = 0.f;
+                for (int j = 0; j < 64; ++j) acc[j] = 0;
                 fence_proxy_async_smem();
             }
         }
@@ -472,26 +480,30 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         // a ring of fewer than three slots has room for a dedicated area
         uint8_t* stg = L.stage_out != kStgAliased ? smem + L.stage_out + warp * kStgWarpBytes
                                                   : smem + (warp / 3) * L.stage_bytes + 2 * kTileBytes + (warp % 3) * kStgWarpBytes;
+        // The flag has been raised in front of the barrier above by whoever gave up: no warp reduces anything then.
+        ok = __all_sync(0xFFFFFFFFu, ok && !*abort_flag);
+        // The rows that a lane reduces (token 4i + lane / 8 of its warp) stay the same for the whole phase.
         const int my_row = valid ? row : p.M;
-        auto reduce_64 = [&](const float (&y)[64], int col0) {
+        uint32_t red_row[8];
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
-                uint32_t w[4];
+        for (int i = 0; i < 8; ++i) red_row[i] = static_cast<uint32_t>(__shfl_sync(0xFFFFFFFFu, my_row, 4 * i + (lane >> 3)));
+        auto pack2 = [](float lo, float hi) {
+            const __nv_bfloat162 h2 = __floats2bfloat162_rn(lo, hi);
+            return *reinterpret_cast<const uint32_t*>(&h2);
+        };
+        auto reduce_64 = [&](const uint32_t (&w)[32], int col0) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    __nv_bfloat162 h2 = __floats2bfloat162_rn(y[8 * g + 2 * i], y[8 * g + 2 * i + 1]);
-                    w[i] = *reinterpret_cast<uint32_t*>(&h2);
-                }
-                *reinterpret_cast<uint4*>(stg + lane * kStgPitch + g * 16) = make_uint4(w[0], w[1], w[2], w[3]);
-            }
+            for (int g = 0; g < 8; ++g)
+                *reinterpret_cast<uint4*>(stg + lane * kStgPitch + g * 16) = make_uint4(w[4 * g], w[4 * g + 1], w[4 * g + 2], w[4 * g + 3]);
             __syncwarp();
+            uint4 vv[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) vv[i] = *reinterpret_cast<const uint4*>(stg + (4 * i + (lane >> 3)) * kStgPitch + (lane & 7) * 16);
+            __nv_bfloat16* base = p.out + col0 + (lane & 7) * 8;
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
-                const int r = 4 * i + (lane >> 3), c = lane & 7;
-                const uint4 v = *reinterpret_cast<const uint4*>(stg + r * kStgPitch + c * 16);
-                const int row_r = __shfl_sync(0xFFFFFFFFu, my_row, r);
-                __nv_bfloat16* dst = p.out + static_cast<size_t>(row_r < p.M ? row_r : 0) * p.K + col0 + c * 8;
-                red_add_v4_bf16x2_raw_if(dst, v, row_r < p.M);
+                const bool live = red_row[i] < static_cast<uint32_t>(p.M);
+                red_add_v4_bf16x2_raw_if(base + static_cast<size_t>(live ? red_row[i] : 0) * p.K, vv[i], live);
             }
             __syncwarp();
         };
@@ -501,42 +513,48 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         // 64 hidden columns: SPC = 2 -> 2 parts of hidden tile jt (columns [0,128) of the buffer are slice 0's
         // partial sums, [128,256) slice 1's); SPC = 1 -> 4 parts covering hidden tiles 2jt and 2jt+1.
         constexpr int PARTS = SPC == 1 ? 4 : 2;
-        for (int jt = 0; jt < ND && ok; ++jt) {
+        for (int jt = hh; jt < ND && ok; jt += 2) {
             const int it = UPI + jt;
             const int b = it & 1;
             const uint32_t aph = (it >> 1) & 1;
-            if ((jt & 1) != hh) continue;
             ok = mbar_wait_warp(&acc_full[b], aph, abort_flag, p.status, 41, it);
             if (!ok) break;
             tc_fence_after();
+            uint32_t va[64], vb[SPC == 2 ? 64 : 1];
+            auto request = [&](int part) {
+                const uint32_t tb = tlane + b * 256 + part * 64;
+#pragma unroll
+                for (int c0 = 0; c0 < 64; c0 += 16) {
+                    tmem_ld16(tb + c0, *reinterpret_cast<uint32_t(*)[16]>(&va[c0]));
+                    if constexpr (SPC == 2) tmem_ld16(tb + 128 + c0, *reinterpret_cast<uint32_t(*)[16]>(&vb[c0]));
+                }
+            };
 #pragma unroll
             for (int part = 0; part < PARTS; ++part) {
                 const int tile = SPC == 1 ? 2 * jt + (part >> 1) : jt;
-                const bool live = warp_valid && tile < KC;
-                float y[64];
-                if (live) {
-                    const uint32_t tb = tlane + b * 256 + part * 64;
+                uint32_t w[32];
+                if (warp_valid) {
+                    request(part);
+                    tmem_ld_wait();
                     if constexpr (SPC == 1) {
-                        uint32_t v[64];
+                        const float f = sw2[min(tile, KC - 1)] * fac[0];
+                        const f32x2 f2 = pack_f32x2(f, f);
 #pragma unroll
-                        for (int c0 = 0; c0 < 64; c0 += 16)
-                            tmem_ld16(tb + c0, *reinterpret_cast<uint32_t(*)[16]>(&v[c0]));
-                        tmem_ld_wait();
-                        const float f = sw2[tile] * fac[0];
-#pragma unroll
-                        for (int e = 0; e < 64; ++e) y[e] = __uint_as_float(v[e]) * f;
-                    } else {
-                        uint32_t va[64], vb[64];
-#pragma unroll
-                        for (int c0 = 0; c0 < 64; c0 += 16) {
-                            tmem_ld16(tb + c0, *reinterpret_cast<uint32_t(*)[16]>(&va[c0]));
-                            tmem_ld16(tb + 128 + c0, *reinterpret_cast<uint32_t(*)[16]>(&vb[c0]));
+                        for (int e = 0; e < 32; ++e) {
+                            float lo, hi;
+                            unpack_f32x2(mul_f32x2(pack_u32x2(va[2 * e], va[2 * e + 1]), f2), lo, hi);
+                            w[e] = pack2(lo, hi);
                         }
-                        tmem_ld_wait();
+                    } else {
                         const float fa = sw2[jt] * fac[0], fb = sw2[KC + jt] * fac[SPC - 1];
+                        const f32x2 fa2 = pack_f32x2(fa, fa), fb2 = pack_f32x2(fb, fb);
 #pragma unroll
-                        for (int e = 0; e < 64; ++e)
-                            y[e] = fmaf(__uint_as_float(va[e]), fa, __uint_as_float(vb[e]) * fb);
+                        for (int e = 0; e < 32; ++e) {
+                            float lo, hi;
+                            unpack_f32x2(fma_f32x2(pack_u32x2(va[2 * e], va[2 * e + 1]), fa2,
+                                                   mul_f32x2(pack_u32x2(vb[2 * e], vb[2 * e + 1]), fb2)), lo, hi);
+                            w[e] = pack2(lo, hi);
+                        }
                     }
                 }
                 if (part == PARTS - 1) {
@@ -545,7 +563,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     __syncwarp();
                     if (lane == 0) mbar_arrive_relaxed_n(&acc_empty[b], 2);   // 4 warps stand in for the barrier's 8
                 }
-                if (live) reduce_64(y, (SPC == 1 ? tile * 128 + (part & 1) * 64 : jt * 128 + part * 64));
+                if (warp_valid && tile < KC) reduce_64(w, SPC == 1 ? tile * 128 + (part & 1) * 64 : jt * 128 + part * 64);
             }
         }
     }
