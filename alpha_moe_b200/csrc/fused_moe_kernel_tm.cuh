@@ -41,6 +41,12 @@ __host__ __device__ inline SmemPlanTm smem_plan_tm(int s, int kc, int spc) {
     p.stage_bytes = 2 * kTileBytes + kTmRows * 128;
     uint32_t o = s * p.stage_bytes;
     p.hq = o;     o += spc * kTmRows * 128;
+    // token scales [K chunk][token]; with four slices they start in the last slice's intermediate, which is written when
+    // they are needed no more
+    if (spc == 4) {
+        p.xs = p.hq + 3 * kTmRows * 128;
+        if (p.xs + kc * kTmRows * 4 > o) o = p.xs + kc * kTmRows * 4;
+    }
     // per epilogue warp a staging tile of 32 rows x 128 B (+16 B pitch padding) for the down phase; with three
     // or more ring slots these live in the slots' token-row tiles, which that phase does not use
     if (s >= 3) { p.stage_out = kStgAliased; } else { p.stage_out = o;  o += 8 * kStgWarpBytes; }
@@ -48,9 +54,9 @@ __host__ __device__ inline SmemPlanTm smem_plan_tm(int s, int kc, int spc) {
     p.swu = o;    o += spc * kc * 4;
     p.sw2 = o;    o += spc * kc * 4;
     o = (o + 15u) & ~15u;
-    p.amaxx = o;  o += 2 * kTmRows * 4;
-    p.xs = o;     o += kc * kTmRows * 4;      // token scales [K chunk][token]
-    p.bars = o;   o += (2 * s + 7) * 8;
+    p.amaxx = o;  o += (spc == 4 ? 4 : 2) * kTmRows * 4;
+    if (spc < 4) { p.xs = o;  o += kc * kTmRows * 4; }
+    p.bars = o;   o += (2 * s + (spc == 4 ? 11 : 7)) * 8;
     p.misc = o;   o += 16;
     p.total = o;
     return p;
@@ -113,7 +119,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     constexpr int W_TMA = 8, W_G0 = 9, W_MMA0 = 10, W_G1 = 12;
     constexpr int GATHER_THREADS = kTmGatherWarps * 32;
     constexpr uint32_t TMEM_COLS = 512;
-    static_assert(SPC == 1 || SPC == 2, "slices per CTA");
+    static_assert(SPC == 1 || SPC == 2 || SPC == 4, "slices per CTA");
 
     const int ngroups = (p.N >> 8) / SPC;
     const int mblock = blockIdx.x / ngroups;
@@ -146,7 +152,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
 
     const int KC = p.K >> 7;
     const int UPI = SPC * KC;
-    const int ND = SPC == 1 ? (KC + 1) >> 1 : KC;
+    const int ND = SPC == 1 ? (KC + 1) >> 1 : SPC / 2 * KC;      // (SPC = 4: two iterations per hidden tile)
     const int NIT = UPI + ND;
     const int S = p.stages;
 
@@ -172,6 +178,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     uint64_t* acc_empty = acc_full + 2;
     uint64_t* h_ready = acc_empty + 2;
     uint64_t* xchg = h_ready + 1;
+    uint64_t* down_full = xchg + 2;      // (four slices) [warpgroup][buffer]: accumulators of a warpgroup's hidden tiles complete
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + L.misc);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(smem + L.misc + 4);
 
@@ -186,6 +193,8 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         }
         mbar_init(h_ready, 1);
         mbar_init(&xchg[0], 8);
+        if (SPC == 4)
+            for (int i = 0; i < 4; ++i) mbar_init(&down_full[i], 1);
         *abort_flag = 0;
         fence_mbar_init();
     }
@@ -214,7 +223,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const uint64_t w_1 = umma_desc_sw128(st0 + kTileBytes);         // its second 128 rows
             const uint64_t x_0 = umma_desc_sw128(st0 + 2 * kTileBytes);     // gathered token rows (M operand)
             const uint64_t h0 = umma_desc_sw128(smem_u32(hq));
-            const uint64_t h1 = umma_desc_sw128(smem_u32(hq + (SPC - 1) * kTmRows * 128));
+            const uint64_t h1 = umma_desc_sw128(smem_u32(hq + (SPC > 1 ? 1 : 0) * kTmRows * 128));
             int s = 0;
             uint32_t ph = 0;
             bool h_waited = false;
@@ -238,9 +247,10 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     } else if (SPC == 1) {
                         umma_f8_chunk1(d, h0, w_0 + off, idesc256);                  // D[token, 2 x 128 hidden rows]
                     } else {
-                        umma_f8_chunk2(d, d + 128, h0, h1, w_0 + off, w_1 + off, idesc128);   // per-slice partial sums
+                        const uint64_t two = SPC == 4 && b ? 2 * kTmRows * 128 / 16 : 0;      // (odd iterations: slices 2 and 3)
+                        umma_f8_chunk2(d, d + 128, h0 + two, h1 + two, w_0 + off, w_1 + off, idesc128);   // per-slice partial sums
                     }
-                    umma_commit(&acc_full[b]);
+                    umma_commit(SPC == 4 && !up ? &down_full[((it - UPI) & 2) + b] : &acc_full[b]);
                     umma_commit(&empty[s]);    // the ring slot is free once these MMAs have read it
                 }
                 __syncwarp();
@@ -269,8 +279,9 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                         tma_load_3d(st, &tm_w2, &full[s], slice0 * 128, (2 * jt) * 128, expert);
                         tma_load_3d(st + kTileBytes, &tm_w2, &full[s], slice0 * 128, (2 * jt + 1) * 128, expert);
                     } else {
-                        tma_load_3d(st, &tm_w2, &full[s], slice0 * 128, jt * 128, expert);
-                        tma_load_3d(st + kTileBytes, &tm_w2, &full[s], (slice0 + 1) * 128, jt * 128, expert);
+                        const int tile = SPC == 4 ? jt >> 1 : jt, first = slice0 + (SPC == 4 ? 2 * (jt & 1) : 0);
+                        tma_load_3d(st, &tm_w2, &full[s], first * 128, tile * 128, expert);
+                        tma_load_3d(st + kTileBytes, &tm_w2, &full[s], (first + 1) * 128, tile * 128, expert);
                     }
                     mbar_arrive_n(&full[s], GATHER_THREADS);
                 }
@@ -435,12 +446,14 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                         acc[8 * g8 + e] = pack_f32x2(h[0], h[1]);
                     }
                 }
-                amaxx[hh * kTmRows + t] = __float_as_uint(amax);
+                // (four slices: two sets of maxima, so that the next slice's are not written before everybody has read these)
+                uint32_t* am = amaxx + (SPC == 4 ? (sl & 1) * 2 * kTmRows : 0);
+                am[hh * kTmRows + t] = __float_as_uint(amax);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&xchg[0]);
                 if (!mbar_wait(&xchg[0], xph, abort_flag, p.status, 42, sl)) ok = false;
                 xph ^= 1;
-                amax = fmaxf(amax, __uint_as_float(amaxx[(hh ^ 1) * kTmRows + t]));
+                amax = fmaxf(amax, __uint_as_float(am[(hh ^ 1) * kTmRows + t]));
                 const float s_h = fmaxf(amax, 1e-10f) * (1.0f / 448.0f);
                 uint8_t* hrow = hq + sl * kTmRows * 128 + t * 128;
 #pragma unroll
@@ -512,6 +525,59 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         // reduction path stays busy.  A warpgroup therefore handles all columns of its iteration, in parts of
         // 64 hidden columns: SPC = 2 -> 2 parts of hidden tile jt (columns [0,128) of the buffer are slice 0's
         // partial sums, [128,256) slice 1's); SPC = 1 -> 4 parts covering hidden tiles 2jt and 2jt+1.
+        if constexpr (SPC == 4) {
+            // A warpgroup takes both iterations of its hidden tile and adds the four slices' partial sums up in registers, so
+            // that a (token, hidden column) is reduced into `out` once per four slices.  Both buffers serve both warpgroups in
+            // turn, and a parity wait must not be two phases off its barrier: each warpgroup has barriers of its own.
+            constexpr int COLS = 32;             // columns of both accumulators per wait (16: 3 % slower, 64 do not fit)
+            for (int jt = hh; jt < KC && ok; jt += 2) {
+                f32x2 y[64];
+#pragma unroll
+                for (int half = 0; half < 2; ++half) {
+                    const int it = UPI + 2 * jt + half;              // UPI is even: buffer `half`
+                    ok = mbar_wait_warp(&down_full[2 * hh + half], (jt >> 1) & 1, abort_flag, p.status, 41, it);
+                    if (!ok) break;
+                    tc_fence_after();
+                    if (warp_valid) {
+                        const float fa = sw2[(2 * half) * KC + jt] * fac[2 * half], fb = sw2[(2 * half + 1) * KC + jt] * fac[2 * half + 1];
+                        const f32x2 fa2 = pack_f32x2(fa, fa), fb2 = pack_f32x2(fb, fb);
+#pragma unroll
+                        for (int c0 = 0; c0 < 128; c0 += COLS) {
+                            uint32_t va[COLS], vb[COLS];
+                            const uint32_t tb = tlane + half * 256 + c0;
+#pragma unroll
+                            for (int c = 0; c < COLS; c += 16) {
+                                tmem_ld16(tb + c, *reinterpret_cast<uint32_t(*)[16]>(&va[c]));
+                                tmem_ld16(tb + 128 + c, *reinterpret_cast<uint32_t(*)[16]>(&vb[c]));
+                            }
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int e = 0; e < COLS / 2; ++e) {
+                                const f32x2 a = pack_u32x2(va[2 * e], va[2 * e + 1]), v = pack_u32x2(vb[2 * e], vb[2 * e + 1]);
+                                f32x2& s = y[c0 / 2 + e];
+                                s = half == 0 ? fma_f32x2(a, fa2, mul_f32x2(v, fb2)) : fma_f32x2(a, fa2, fma_f32x2(v, fb2, s));
+                            }
+                        }
+                    }
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive_relaxed_n(&acc_empty[half], 2);
+                }
+                if (ok && warp_valid) {
+#pragma unroll
+                    for (int part = 0; part < 2; ++part) {
+                        uint32_t w[32];
+#pragma unroll
+                        for (int e = 0; e < 32; ++e) {
+                            float lo, hi;
+                            unpack_f32x2(y[32 * part + e], lo, hi);
+                            w[e] = pack2(lo, hi);
+                        }
+                        reduce_64(w, jt * 128 + part * 64);
+                    }
+                }
+            }
+        } else {
         constexpr int PARTS = SPC == 1 ? 4 : 2;
         for (int jt = hh; jt < ND && ok; jt += 2) {
             const int it = UPI + jt;
@@ -565,6 +631,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                 }
                 if (warp_valid && tile < KC) reduce_64(w, SPC == 1 ? tile * 128 + (part & 1) * 64 : jt * 128 + part * 64);
             }
+        }
         }
     }
 

@@ -161,6 +161,21 @@ int plan(int K, int block_m, int stages, int spc, int ksplit, int* depth, int* b
     return fail(ALPHA_MOE_E_ARG, "K=%d block_m=%d does not fit in shared memory even with one stage", K, block_m);
 }
 
+// Slices of the intermediate dimension per CTA.  block_n = 64 asks for the wide variant: one CTA owns two 128-column slices
+// (one reduction per token and expert instead of two); it needs an even slice count.
+// Blocks above 64 have a form with four slices per CTA, which halves the reductions once more and the number of times that
+// token rows and scales are set up.  It is taken where its CTAs still make three rounds (fewer, and the last round, partly
+// filled, costs what it saves) and its ring keeps the asked-for depth up to three.  Unsharded layer (16 slices), calls in a
+// row, two slices and four: M = 4096 3767 and 3604 us, M = 3000 2851 and 2745, M = 2048 (Zipf) 3081 and 2916, M = 1700 2540
+// and 2511.
+int slices_per_cta(int K, int N, int block_m, int block_n, int stages, long long nblocks, int sms) {
+    const int slices = N / 256;
+    if (block_n != 64 || slices % 2 != 0) return 1;
+    if (!token_major(block_m) || slices % 4 != 0 || nblocks * (slices / 4) < 3LL * sms) return 2;
+    const int kc = K / 128, want = std::min(stages, 3);
+    return static_cast<int>(amoe::smem_plan_tm(want, kc, 4).total) <= kMaxDynSmem ? 4 : 2;
+}
+
 // Opts a kernel into the large dynamic shared-memory window once per device (atomically: several host threads
 // may launch at the same time).
 template <typename Kern>
@@ -670,12 +685,10 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     DeviceFacts facts;
     if (int rc = device_facts(dev, &facts)) return rc;
 
-    // block_n = 64 asks for the wide variant: one CTA owns two 128-column slices of the intermediate
-    // dimension (one reduction per token and expert instead of two); it needs an even slice count.
-    const int spc = (block_n == 64 && (N / 256) % 2 == 0) ? 2 : 1;
     // Live blocks never exceed the number of assignments, so no more CTAs than that are launched.
     long long nblocks = (static_cast<long long>(sorted_num) + block_m - 1) / block_m;
     if (nblocks > static_cast<long long>(M) * top_k) nblocks = static_cast<long long>(M) * top_k;
+    const int spc = slices_per_cta(K, N, block_m, block_n, stages, nblocks, facts.sms);
     const int ksplit = choose_ksplit(block_m, spc, nblocks, N, K, stages, facts.clusters);
     int depth, bmp, smem_bytes;
     if (int rc = plan(K, block_m, stages, spc, ksplit, &depth, &bmp, &smem_bytes)) return rc;
@@ -721,7 +734,8 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     const bool pair64 = bmp == 64 && depth <= 2 && smem_bytes <= kPairDynSmem;
     if (token_major(block_m))
         return spc == 1 ? launch_tokmajor<1>(maps, p, g, smem_bytes, dev, st)
-                        : launch_tokmajor<2>(maps, p, g, smem_bytes, dev, st);
+             : spc == 2 ? launch_tokmajor<2>(maps, p, g, smem_bytes, dev, st)
+                        : launch_tokmajor<4>(maps, p, g, smem_bytes, dev, st);
     if (tp_world > 1) {       // the form that adds into the peers' buffers: one shape per tile width
         if (spc == 1) {
             switch (bmp) {
@@ -943,7 +957,6 @@ int alpha_moe_b200_plan(int K, int N, int block_m, int block_n, int stages, int 
     if (block_n != 32 && block_n != 64) return fail(ALPHA_MOE_E_ARG, "block_n must be 32 or 64, got %d", block_n);
     if (stages < 1 || stages > 5) return fail(ALPHA_MOE_E_ARG, "stages must be in 1..5, got %d", stages);
     if (num_blocks <= 0 || num_sms < 0) return fail(ALPHA_MOE_E_ARG, "num_blocks must be positive, num_sms >= 0");
-    const int spc = (block_n == 64 && (N / 256) % 2 == 0) ? 2 : 1;
     ClusterCapacity clusters;
     if (num_sms == 0) {           // the current device, as a launch would see it
         int dev = 0;
@@ -954,6 +967,7 @@ int alpha_moe_b200_plan(int K, int N, int block_m, int block_n, int stages, int 
     } else {
         model_cluster_capacity(num_sms, &clusters);
     }
+    const int spc = slices_per_cta(K, N, block_m, block_n, stages, 0, 1);      // (one or two: see the header)
     const int ksplit = choose_ksplit(block_m, spc, num_blocks, N, K, stages, clusters);
     int depth, bmp, smem_bytes;
     if (int rc = plan(K, block_m, stages, spc, ksplit, &depth, &bmp, &smem_bytes)) return rc;

@@ -34,7 +34,8 @@ extern "C" {
  * reference's tuning knobs and are validated like csrc/torch_interface.cpp:62-64:
  * (block_n,warp_n) in {(64,4),(32,8)}, 1 <= stages <= 5, block_m in {8,16,...,128}.
  * Here stages = depth of the shared-memory ring (lowered if it would not fit), and block_n = 64
- * selects the variant in which one CTA owns two 128-column slices of the intermediate dimension.
+ * selects the variant in which one CTA owns two 128-column slices of the intermediate dimension (four, with
+ * block_m > 64, N/256 a multiple of four and blocks for several rounds of CTAs).
  * Requires K % 128 == 0, N % 256 == 0, 16-byte aligned w / w2 / x; `out` 4-byte aligned for block_m <= 64 and
  * 16-byte aligned for block_m > 64 (those kernels accumulate with 16-byte vector reductions). */
 int alpha_moe_b200_fused_moe_w8a8_up_down(
@@ -198,7 +199,8 @@ int alpha_moe_b200_selftest_warp_wait(int limit_cycles, int32_t* result5, void* 
  * num_sms = SM count of a device (148 on B200): the cluster capacity that decides ksplit is then modelled (GPCs of
  * about 18 SMs; one CTA per SM, two when the ring is shallow enough for two to share an SM) and nothing touches a
  * device; num_sms = 0 = the current device, whose driver is asked as a launch would (launches nothing).  out6 = {ring_depth, padded_block_m, dynamic_smem_bytes,
- * slices_per_cta (2 when block_n = 64 and N/256 is even), ksplit (CTAs per cluster along K, small batches: the
+ * slices_per_cta (2 when block_n = 64 and N/256 is even; large launches that put two such pairs into one CTA are
+ * planned as the pairs), ksplit (CTAs per cluster along K, small batches: the
  * largest of 2..8 for which all (block, slice) units get their cluster at the same time, else 1),
  * kernel (0 weight-major, 1 token-major)}. */
 int alpha_moe_b200_plan(int K, int N, int block_m, int block_n, int stages, int num_blocks, int num_sms,

@@ -367,3 +367,17 @@ def test_token_major_scale_staging(k, inter, m, bm, stages, offset):
     d["x_scale"] = buf[offset:].view(case.x_scale.shape)
     d["x_scale"].copy_(case.x_scale)
     check_close(run_capi(case, bm, 64, 4, stages, dcase=d), orc.run_oracle(case, bm), tag=f"k={k} bm={bm} off={offset}")
+
+
+@pytest.mark.parametrize("k,inter,m,top_k,bm,stages", [
+    (128, 4096, 1010, 4, 72, 3),      # a single hidden tile: the second warpgroup has none
+    (384, 4096, 1010, 4, 72, 1),      # three hidden tiles, one ring slot
+    (256, 4096, 1800, 4, 128, 2),     # two ring slots: staging tiles of their own
+    (640, 4096, 1800, 4, 128, 5),     # five tiles, scale rows that are not multiples of 16 bytes
+])
+def test_four_slices_per_cta(k, inter, m, top_k, bm, stages):
+    """Blocks above 64 with an intermediate size that is a multiple of 512, and enough blocks for three rounds of CTAs.  Bounds as
+    above."""
+    case = orc.make_case(6, k, inter, m, top_k, seed=k + m, scaling=1.5)
+    assert m * top_k // bm * (inter // 512) >= 3 * 148
+    check_close(run_capi(case, bm, 64, 4, stages), orc.run_oracle(case, bm), tag=f"k={k} I={inter} bm={bm}")
