@@ -21,7 +21,8 @@
 // Ring slot: [256 weight rows x 128 B = 32 KB][128 token rows x 128 B = 16 KB]; slot contents as in
 // fused_moe_kernel.cuh.  TMEM: up phase two buffers of 256 columns (one per K chunk in flight); down
 // phase two buffers of 256 columns (SPC = 1: two hidden tiles; SPC = 2: the two slices' partial sums
-// of one hidden tile, combined by the epilogue because each carries its own scales).
+// of one hidden tile, combined by the epilogue because each carries its own scales; SPC = 4: slices 0 and 1 of a
+// hidden tile, then 2 and 3).
 #pragma once
 
 #include "fused_moe_kernel.cuh"
@@ -370,9 +371,9 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         // Accumulators of this token: 8 groups of (8 gate, 8 up) columns = 64 intermediate columns, as packed pairs.  In a row
         // of calls this kernel runs at the power limit, where an instruction saved counts even if its unit was not busy.  Packed
         // FMAs, the rows of the down phase's reductions in registers instead of a shuffle and a 64-bit multiplication for each,
-        // no vote per chunk and one issuing warp instead of two that took turns: DeepSeek-V3 TP8 shard, M = 4096 535 -> 514 us,
-        // M = 8192 (Zipf) 887 -> 846, unsharded M = 4096 4015 -> 3886, Qwen3-Next shard M = 4096 233 -> 220 (the rows alone
-        // are two thirds of it).  For the same reason token rows of padding stay zero: left as they are, M = 4096 is 3 % slower.
+        // no vote per chunk and one issuing warp instead of two that took turns: DeepSeek-V3 TP8 shard, M = 4096 531 -> 507 us,
+        // M = 8192 (Zipf) 885 -> 854, unsharded M = 4096 3915 -> 3744, Qwen3-Next shard M = 4096 230 -> 220 (the rows alone
+        // are two thirds of it).  For the same reason token rows of padding are zeroed: left as they are, M = 4096 is 3 % slower.
         f32x2 acc[64];
 #pragma unroll
         for (int j = 0; j < 64; ++j) acc[j] = 0;
