@@ -37,6 +37,13 @@ constexpr uint32_t kStgAliased = 0xFFFFFFFFu;      // SmemPlanTm::stage_out when
 struct SmemPlanTm {
     uint32_t stage_bytes, hq, stage_out, swg, swu, sw2, amaxx, xs, bars, misc, total;
 };
+// Row maxima of consecutive slices go to two sets of words in turn where nothing else keeps a warp from writing the next
+// slice's before its partner has read this one's.  With two accumulator buffers a warp ends a slice only when every warp has
+// released the slice's third chunk from the end, so from three chunks a slice on that is a chunk of the same slice, which the
+// partner released after it read the maxima before.  (With two slices and more chunks a second set would be 1 KB that the
+// largest accepted hidden size lacks.)
+__host__ __device__ constexpr bool two_sets_of_maxima(int spc, int kc) { return spc == 4 || (spc == 2 && kc <= 2); }
+
 __host__ __device__ inline SmemPlanTm smem_plan_tm(int s, int kc, int spc) {
     SmemPlanTm p;
     p.stage_bytes = 2 * kTileBytes + kTmRows * 128;
@@ -55,7 +62,7 @@ __host__ __device__ inline SmemPlanTm smem_plan_tm(int s, int kc, int spc) {
     p.swu = o;    o += spc * kc * 4;
     p.sw2 = o;    o += spc * kc * 4;
     o = (o + 15u) & ~15u;
-    p.amaxx = o;  o += (spc == 4 ? 4 : 2) * kTmRows * 4;
+    p.amaxx = o;  o += (two_sets_of_maxima(spc, kc) ? 4 : 2) * kTmRows * 4;
     if (spc < 4) { p.xs = o;  o += kc * kTmRows * 4; }
     p.bars = o;   o += (2 * s + (spc == 4 ? 11 : 7)) * 8;
     p.misc = o;   o += 16;
@@ -171,7 +178,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     float* swg = reinterpret_cast<float*>(smem + L.swg);
     float* swu = reinterpret_cast<float*>(smem + L.swu);
     float* sw2 = reinterpret_cast<float*>(smem + L.sw2);
-    uint32_t* amaxx = reinterpret_cast<uint32_t*>(smem + L.amaxx);    // [2][128] per-thread |h| maxima of each column half
+    uint32_t* amaxx = reinterpret_cast<uint32_t*>(smem + L.amaxx);    // one or two sets of [2][128] per-thread |h| maxima of each column half
     float* xs = reinterpret_cast<float*>(smem + L.xs);                // [KC][128] token scales (0 for padding rows)
     uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bars);
     uint64_t* empty = full + S;
@@ -447,8 +454,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                         acc[8 * g8 + e] = pack_f32x2(h[0], h[1]);
                     }
                 }
-                // (four slices: two sets of maxima, so that the next slice's are not written before everybody has read these)
-                uint32_t* am = amaxx + (SPC == 4 ? (sl & 1) * 2 * kTmRows : 0);
+                uint32_t* am = amaxx + (two_sets_of_maxima(SPC, KC) ? (sl & 1) * 2 * kTmRows : 0);
                 am[hh * kTmRows + t] = __float_as_uint(amax);
                 __syncwarp();
                 if (lane == 0) mbar_arrive(&xchg[0]);

@@ -145,6 +145,25 @@ def test_largest_hidden_size_that_fits_a_ring_of_one_slot(block_m, block_n, larg
         capi.plan(largest + 128, block_m, 5, block_n)
 
 
+def test_row_maxima_of_two_slices_share_memory_only_where_their_uses_are_ordered():
+    """Token-major kernel, two slices of kc chunks each, two accumulator buffers: the UMMAs of chunk i wait until every
+    epilogue warp has released chunk i - 2.  A warp reads its partner's maxima of the first slice after it has released chunk
+    kc - 1 and before it releases chunk kc; another warp writes those of the second slice once chunk 2 kc - 1 is complete.
+    Unless the release of 2 kc - 3, which that chunk waits for, lies behind the read, both slices need words of their own."""
+    from alpha_moe_b200 import capi
+
+    def plan_bytes(kc):
+        return capi.plan(128 * kc, 128, 3, 64, N=512)[2]
+
+    def without_maxima(kc):       # what grows with kc: block scales (padded to 16 bytes) and token scales
+        return (3 * 2 * kc * 4 + 15) // 16 * 16 + 512 * kc
+
+    one_set = plan_bytes(8) - without_maxima(8)
+    for kc in range(1, 8):
+        ordered = 2 * kc - 3 >= kc
+        assert plan_bytes(kc) - without_maxima(kc) == one_set + (0 if ordered else 2 * 128 * 4), kc
+
+
 def test_out_alignment_is_checked_per_kernel_before_anything_is_launched():
     """block_m > 64 accumulates with 16-byte vector reductions: an `out` that is only 4-byte aligned must be
     rejected with an argument error (it would fault on the device); block_m <= 64 accepts it.  The call with
