@@ -164,14 +164,18 @@ int plan(int K, int block_m, int stages, int spc, int ksplit, int* depth, int* b
 // Slices of the intermediate dimension per CTA.  block_n = 64 asks for the wide variant: one CTA owns two 128-column slices
 // (one reduction per token and expert instead of two); it needs an even slice count.
 // Blocks above 64 have a form with four slices per CTA, which halves the reductions once more and the number of times that
-// token rows and scales are set up.  It is taken where its CTAs still make three rounds (fewer, and the last round, partly
-// filled, costs what it saves) and its ring keeps the asked-for depth up to three.  Unsharded layer (16 slices), calls in a
-// row, two slices and four: M = 4096 3767 and 3604 us, M = 3000 2851 and 2745, M = 2048 (Zipf) 3081 and 2916, M = 1700 2540
-// and 2511.
-int slices_per_cta(int K, int N, int block_m, int block_n, int stages, long long nblocks, int sms) {
+// token rows and scales are set up, but also the number of CTAs.  It is taken where at least three rounds of them are live
+// however the routing falls: live_min = the fewest blocks that can hold the batch (the blocks a schedule has room for are up to
+// one per expert more, so they say nothing).  With fewer rounds the last one, partly filled, can cost more than the form saves.
+// Operator, calls in a row, four slices against two, by live_min's rounds, over uniform and Zipf routing and one set of experts
+// for all tokens (K = 7168, I = 512 / 1024 / 2048, 1200-8192 tokens; K = 2048, I = 512 / 1024, 3600-8192 tokens): three and
+// more 0.86-1.00 (unsharded DeepSeek-V3 layer, M = 4096 3602 and 3452 us, Zipf 3758 and 3482; M = 1200 2239 and
+// 2240); two to three 0.87-1.02; below two 0.87-1.18 (I = 512, M = 2048: uniform 635 and 595, Zipf 729 and 796, one set of
+// experts 391 and 435).  The ring must keep the asked-for depth up to three.
+int slices_per_cta(int K, int N, int block_m, int block_n, int stages, long long live_min, int sms) {
     const int slices = N / 256;
     if (block_n != 64 || slices % 2 != 0) return 1;
-    if (!token_major(block_m) || slices % 4 != 0 || nblocks * (slices / 4) < 3LL * sms) return 2;
+    if (!token_major(block_m) || slices % 4 != 0 || live_min * (slices / 4) < 3LL * sms) return 2;
     const int kc = K / 128, want = std::min(stages, 3);
     return static_cast<int>(amoe::smem_plan_tm(want, kc, 4).total) <= kMaxDynSmem ? 4 : 2;
 }
@@ -688,7 +692,8 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     // Live blocks never exceed the number of assignments, so no more CTAs than that are launched.
     long long nblocks = (static_cast<long long>(sorted_num) + block_m - 1) / block_m;
     if (nblocks > static_cast<long long>(M) * top_k) nblocks = static_cast<long long>(M) * top_k;
-    const int spc = slices_per_cta(K, N, block_m, block_n, stages, nblocks, facts.sms);
+    const long long live_min = std::min(nblocks, (static_cast<long long>(M) * top_k + block_m - 1) / block_m);
+    const int spc = slices_per_cta(K, N, block_m, block_n, stages, live_min, facts.sms);
     const int ksplit = choose_ksplit(block_m, spc, nblocks, N, K, stages, facts.clusters);
     int depth, bmp, smem_bytes;
     if (int rc = plan(K, block_m, stages, spc, ksplit, &depth, &bmp, &smem_bytes)) return rc;

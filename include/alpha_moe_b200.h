@@ -35,7 +35,7 @@ extern "C" {
  * (block_n,warp_n) in {(64,4),(32,8)}, 1 <= stages <= 5, block_m in {8,16,...,128}.
  * Here stages = depth of the shared-memory ring (lowered if it would not fit), and block_n = 64
  * selects the variant in which one CTA owns two 128-column slices of the intermediate dimension (four, with
- * block_m > 64, N/256 a multiple of four and blocks for several rounds of CTAs).
+ * block_m > 64, N/256 a multiple of four and ceil(M * top_k / block_m) blocks for three rounds of CTAs).
  * Requires K % 128 == 0, N % 256 == 0, 16-byte aligned w / w2 / x; `out` 4-byte aligned for block_m <= 64 and
  * 16-byte aligned for block_m > 64 (those kernels accumulate with 16-byte vector reductions). */
 int alpha_moe_b200_fused_moe_w8a8_up_down(

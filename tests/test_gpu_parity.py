@@ -7,6 +7,7 @@ same seeded inputs.  Tolerances (floating point, bf16 output accumulated with at
 """
 import dataclasses
 import os
+import re
 
 import numpy as np
 import pytest
@@ -367,6 +368,30 @@ def test_token_major_scale_staging(k, inter, m, bm, stages, offset):
     d["x_scale"] = buf[offset:].view(case.x_scale.shape)
     d["x_scale"].copy_(case.x_scale)
     check_close(run_capi(case, bm, 64, 4, stages, dcase=d), orc.run_oracle(case, bm), tag=f"k={k} bm={bm} off={offset}")
+
+
+def slices_launched(call):
+    """Slices per CTA of the one token-major kernel that `call` launches (the template argument in the kernel's name)."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        call()
+        torch.cuda.synchronize()
+    found = [mt.group(1) for mt in (re.search(r"tokmajor_kernel<(\d)>", e.key) for e in prof.key_averages()) if mt]
+    assert len(found) == 1, [e.key for e in prof.key_averages()]
+    return int(found[0])
+
+
+def test_empty_blocks_of_a_schedule_do_not_count_as_rounds_of_four_slice_ctas():
+    """512 experts of which two get all 1200 assignments: the schedule has room for more than 444 blocks, 18 are live."""
+    case = orc.make_case(512, 128, 512, 600, 2, seed=3)
+    case = dataclasses.replace(case, topk_ids=torch.tensor([[3, 500]], dtype=case.topk_ids.dtype).repeat(600, 1))
+    sid, _, npp = case.schedule(72)
+    assert int(npp) == 18 * 72
+    assert sid.numel() // 72 >= 3 * 148
+    dcase = to_device(case)
+    got = []
+    assert slices_launched(lambda: got.append(run_capi(case, 72, 64, 4, 3, dcase=dcase))) == 2
+    check_close(got[0], orc.run_oracle(case, 72), tag="few live blocks")
 
 
 @pytest.mark.parametrize("k,inter,m,top_k,bm,stages", [
