@@ -963,16 +963,19 @@ int alpha_moe_b200_plan(int K, int N, int block_m, int block_n, int stages, int 
     if (stages < 1 || stages > 5) return fail(ALPHA_MOE_E_ARG, "stages must be in 1..5, got %d", stages);
     if (num_blocks <= 0 || num_sms < 0) return fail(ALPHA_MOE_E_ARG, "num_blocks must be positive, num_sms >= 0");
     ClusterCapacity clusters;
+    int sms = num_sms;
     if (num_sms == 0) {           // the current device, as a launch would see it
         int dev = 0;
         CUDA_TRY(cudaGetDevice(&dev));
         DeviceFacts facts;
         if (int rc = device_facts(dev, &facts)) return rc;
         clusters = facts.clusters;
+        sms = facts.sms;
     } else {
         model_cluster_capacity(num_sms, &clusters);
     }
-    const int spc = slices_per_cta(K, N, block_m, block_n, stages, 0, 1);      // (one or two: see the header)
+    // (one count is enough: blocks that can be split along K are not those that can take four slices)
+    const int spc = slices_per_cta(K, N, block_m, block_n, stages, num_blocks, sms);
     const int ksplit = choose_ksplit(block_m, spc, num_blocks, N, K, stages, clusters);
     int depth, bmp, smem_bytes;
     if (int rc = plan(K, block_m, stages, spc, ksplit, &depth, &bmp, &smem_bytes)) return rc;

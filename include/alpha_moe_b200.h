@@ -195,14 +195,15 @@ int alpha_moe_b200_selftest_wait_timeout(int limit_cycles, int where, int iter, 
 int alpha_moe_b200_selftest_warp_wait(int limit_cycles, int32_t* result5, void* stream);
 
 /* What the launcher uses for a problem and a knob tuple; for tuners and tests.  It runs the launcher's own
- * planning code.  num_blocks = live upper bound of schedule blocks, min(ceil(sorted_num / block_m), M * top_k);
+ * planning code.  num_blocks = schedule blocks as the launcher counts them: for block_m <= 64 those that can be live at most,
+ * min(ceil(sorted_num / block_m), M * top_k), which decide ksplit; for block_m > 64 those that are live at least,
+ * min(ceil(sorted_num / block_m), ceil(M * top_k / block_m)), which decide slices_per_cta;
  * num_sms = SM count of a device (148 on B200): the cluster capacity that decides ksplit is then modelled (GPCs of
  * about 18 SMs; one CTA per SM, two when the ring is shallow enough for two to share an SM) and nothing touches a
  * device; num_sms = 0 = the current device, whose driver is asked as a launch would (launches nothing).  out6 = {ring_depth, padded_block_m, dynamic_smem_bytes,
- * slices_per_cta (2 when block_n = 64 and N/256 is even; large launches that put two such pairs into one CTA are
- * planned as the pairs), ksplit (CTAs per cluster along K, small batches: the
- * largest of 2..8 for which all (block, slice) units get their cluster at the same time, else 1),
- * kernel (0 weight-major, 1 token-major)}. */
+ * slices_per_cta (2 when block_n = 64 and N/256 is even, 4 in large launches as said above, else 1), ksplit (CTAs per
+ * cluster along K, small batches: the largest of 2..8 for which all (block, slice) units get their cluster at the same
+ * time, else 1), kernel (0 weight-major, 1 token-major)}. */
 int alpha_moe_b200_plan(int K, int N, int block_m, int block_n, int stages, int num_blocks, int num_sms,
                         int32_t* out6);
 

@@ -116,7 +116,10 @@ def test_plan_fits_shared_memory_for_every_knob():
                             depth, bmp, smem, spc, ks, kern = capi.plan(k, bm, st, bn, N=n, num_blocks=nblocks)
                             assert 1 <= depth <= st and bmp >= bm and bmp in (16, 32, 64, 128)
                             assert smem <= 232448
-                            assert spc == (2 if bn == 64 and (n // 256) % 2 == 0 else 1)
+                            # 600 blocks are three rounds of 148 CTAs with four of the 16 slices each; every ring of up to
+                            # three slots fits beside them at these hidden sizes
+                            four = bm > 64 and bn == 64 and (n // 256) % 4 == 0 and nblocks * (n // 1024) >= 3 * 148
+                            assert spc == (4 if four else 2 if bn == 64 and (n // 256) % 2 == 0 else 1)
                             assert kern == (0 if bm <= 64 else 1)
                             assert 1 <= ks <= min(8, k // 128) and (ks == 1 or (bm <= 32 and spc == 1 and nblocks == 9))
     assert capi.plan(7168, 16, 5)[0] == 5
@@ -143,6 +146,28 @@ def test_largest_hidden_size_that_fits_a_ring_of_one_slot(block_m, block_n, larg
     assert capi.plan(largest, block_m, 5, block_n)[0] == 1
     with pytest.raises(capi.AlphaMoeError, match="does not fit"):
         capi.plan(largest + 128, block_m, 5, block_n)
+
+
+@pytest.mark.parametrize("k", [128, 2048, 4096, 4224, 7168])
+def test_four_slice_plans(k):
+    """Four slices per CTA: at three rounds of CTAs and not below, and only with the ring depth asked for, up to three.  The token
+    scales start in the last slice's intermediate (16 KB, which 32 chunks fill) and the staging area stands alone below three
+    slots."""
+    from alpha_moe_b200 import capi
+    kc = k // 128
+    for st in range(1, 6):
+        assert capi.plan(k, 128, st, 64, N=1024, num_blocks=443)[3] == 2
+        depth, bmp, smem, spc, ks, kern = capi.plan(k, 128, st, 64, N=1024, num_blocks=444)
+        assert (spc, ks, kern, bmp) == (4, 1, 1, 128)
+        ring = 48 * 1024 * depth + (0 if depth >= 3 else 8 * 32 * 144)
+        maxima, scales = 4 * 128 * 4, (3 * 4 * kc * 4 + 15) // 16 * 16
+        barriers = 8 * (2 * depth + 11) + 16
+        assert smem == ring + 4 * 16384 + max(0, 512 * kc - 16384) + scales + maxima + barriers <= 232448
+        assert depth == min(st, 3)
+    assert capi.plan(k, 128, 3, 64, N=512, num_blocks=1 << 20)[3] == 2          # two slices in all
+    assert capi.plan(k, 128, 3, 32, N=1024, num_blocks=1 << 20)[3] == 1
+    assert capi.plan(k, 64, 3, 64, N=1024, num_blocks=1 << 20)[3] == 2          # the other kernel
+    assert capi.plan(26752, 128, 3, 64, N=1024, num_blocks=1 << 20)[3] == 2     # such a ring would not fit
 
 
 def test_row_maxima_of_two_slices_share_memory_only_where_their_uses_are_ordered():
