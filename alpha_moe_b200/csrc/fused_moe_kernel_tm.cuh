@@ -84,7 +84,7 @@ __device__ __forceinline__ void stage_token_scales(float* xs, const float* row, 
 #pragma unroll
             for (int i = 0; i < BATCH; ++i) {
                 const int u = u0 + i * step;
-                v[i] = live && u < units ? __ldg(reinterpret_cast<const float4*>(row) + u) : make_float4(0.f, 0.f, 0.f, 0.f);
+                v[i] = live && u < units ? reinterpret_cast<const float4*>(row)[u] : make_float4(0.f, 0.f, 0.f, 0.f);
             }
 #pragma unroll
             for (int i = 0; i < BATCH; ++i) {
@@ -103,7 +103,7 @@ __device__ __forceinline__ void stage_token_scales(float* xs, const float* row, 
 #pragma unroll
             for (int i = 0; i < BATCH; ++i) {
                 const int u = u0 + i * step;
-                v[i] = live && u < units ? __ldg(row + u) : 0.f;
+                v[i] = live && u < units ? row[u] : 0.f;
             }
 #pragma unroll
             for (int i = 0; i < BATCH; ++i)
@@ -142,8 +142,8 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     int pid_pre[MAXG];
     int expert;
     {
-        const int npad_raw = ld_global_nc_s32(p.num_tokens_post_padded);
-        expert = ld_global_nc_s32(p.expert_ids + mblock);
+        const int npad_raw = ld_global_s32(p.num_tokens_post_padded);
+        expert = ld_global_s32(p.expert_ids + mblock);
         const bool gather_role = warp == W_G0 || warp >= W_G1;
 #pragma unroll
         for (int i = 0; i < MAXG; ++i) {
@@ -152,7 +152,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
             const int idx = mblock * p.block_m + row;
             pid_pre[i] = -1;
             if ((gather_role || (i == 0 && warp < W_TMA)) && row < p.block_m && idx < p.sorted_num)
-                pid_pre[i] = ld_global_nc_s32(p.sorted_token_ids + idx);
+                pid_pre[i] = ld_global_s32(p.sorted_token_ids + idx);
         }
         if (mblock * p.block_m >= min(npad_raw, p.sorted_num)) return;
         if (expert < 0 || expert >= p.E) return;

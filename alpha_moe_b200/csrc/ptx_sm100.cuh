@@ -431,11 +431,12 @@ template <int N>
 __device__ __forceinline__ void setmaxnreg_dec() {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
-// Read-only global load that the compiler keeps where it is written (used to request small schedule words
-// at kernel entry, ahead of the set-up work whose latency they then overlap).
-__device__ __forceinline__ int ld_global_nc_s32(const int* p) {
+// Global load that the compiler keeps where it is written (used to request small schedule words at kernel entry, ahead of the
+// set-up work whose latency they then overlap).  Not ld.global.nc or __ldg, which want memory that nothing writes while the
+// kernel runs: as a programmatic dependent it is there before the kernel in front has written them.
+__device__ __forceinline__ int ld_global_s32(const int* p) {
     int v;
-    asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
 // Programmatic dependent launch.  A kernel launched with the programmatic-serialisation attribute may start while

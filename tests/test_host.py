@@ -189,6 +189,18 @@ def test_row_maxima_of_two_slices_share_memory_only_where_their_uses_are_ordered
         assert plan_bytes(kc) - without_maxima(kc) == one_set + (0 if ordered else 2 * 128 * 4), kc
 
 
+def test_no_kernel_reads_through_the_non_coherent_path():
+    """The fused and exchange kernels are launched as programmatic dependents: they may be running while the kernel that
+    writes their schedule, scales and activations still is.  ld.global.nc and __ldg are defined only for memory that nothing
+    writes while the kernel runs, and const __restrict__ pointers let the compiler choose them."""
+    src = os.path.join(ROOT, "alpha_moe_b200", "csrc")
+    for name in os.listdir(src):
+        if name.endswith((".cu", ".cuh")):
+            with open(os.path.join(src, name)) as f:
+                code = re.sub(r"//[^\n]*", "", f.read())
+            assert not re.search(r"\.nc\b|__ldg|__restrict__", code), name
+
+
 def test_out_alignment_is_checked_per_kernel_before_anything_is_launched():
     """block_m > 64 accumulates with 16-byte vector reductions: an `out` that is only 4-byte aligned must be
     rejected with an argument error (it would fault on the device); block_m <= 64 accepts it.  The call with
