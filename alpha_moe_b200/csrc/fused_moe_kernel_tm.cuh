@@ -481,7 +481,16 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
                     const int chunk = (hh * 4 + i) ^ (t & 7);
                     *reinterpret_cast<uint4*>(hrow + chunk * 16) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
                 }
-                fac[sl] = s_h * tw * p.scaling;
+                // The loop over slices is not unrolled, and an index that varies puts the array on the stack: two are told apart
+                // instead (DeepSeek-V3 TP8 shard, M = 4096 515 -> 513 us, M = 8192 (Zipf) 856 -> 847).  Four stay there, one
+                // load each per hidden tile: kept in registers they make 176 bytes of spills out of 32.
+                const float f = s_h * tw * p.scaling;
+                if constexpr (SPC == 2) {
+                    if (sl == 0) fac[0] = f;
+                    else fac[SPC - 1] = f;
+                } else {
+                    fac[sl] = f;
+                }
 #pragma unroll
                 for (int j = 0; j < 64; ++j) acc[j] = 0;
                 fence_proxy_async_smem();
