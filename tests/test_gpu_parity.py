@@ -356,7 +356,8 @@ def test_reference_timing_scripts_imbalance_model(balancedness):
     (128, 256, 130, 128, 3),      # a single K chunk: no warpgroup has a second one to stage
     (384, 256, 300, 96, 1),       # three chunks: the scale rows are not multiples of 16 bytes; one ring slot
     (512, 128, 257, 128, 2),      # four chunks, one slice per CTA
-    (4608, 256, 200, 72, 4),      # 36 chunks: more 16-byte pieces than one batch of loads
+    (4608, 256, 200, 72, 4),      # 36 chunks: one batch of 16-byte loads, several of single ones
+    (8704, 128, 150, 72, 2),      # 68 chunks, 17 pieces: one warpgroup has a second batch of one piece, the other none
 ])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_token_major_scale_staging(k, inter, m, bm, stages, offset):
@@ -405,4 +406,32 @@ def test_four_slices_per_cta(k, inter, m, top_k, bm, stages):
     above."""
     case = orc.make_case(6, k, inter, m, top_k, seed=k + m, scaling=1.5)
     assert m * top_k // bm * (inter // 512) >= 3 * 148
-    check_close(run_capi(case, bm, 64, 4, stages), orc.run_oracle(case, bm), tag=f"k={k} I={inter} bm={bm}")
+    dcase = to_device(case)
+    got = []
+    assert slices_launched(lambda: got.append(run_capi(case, bm, 64, 4, stages, dcase=dcase))) == 4
+    check_close(got[0], orc.run_oracle(case, bm), tag=f"k={k} I={inter} bm={bm}")
+
+
+@pytest.mark.parametrize("k", [4096, 4224, 7168])
+@pytest.mark.parametrize("m,slices", [(3996, 4), (3987, 2)])
+def test_four_slices_are_a_whole_block(k, m, slices):
+    """512 intermediate columns: one CTA per block, at 444 blocks of 72, not at 443.  The token scales fill the last slice's
+    intermediate (k = 4096), go beyond it by one chunk and by 24.  The schedule is cut to three live blocks, a full one, an
+    expert's last one and another full one, so that the oracle stays quick; rows of other tokens must stay zero."""
+    bm = 72
+    case = orc.make_case(8, k, 512, m, 8, seed=k, scaling=1.5)
+    sid, eid, npp = case.schedule(bm)
+    live = eid[:int(npp) // bm].tolist()
+    pick = [live.index(2), len(live) - 1 - live[::-1].index(5), live.index(7)]
+    for i, b in enumerate(pick):
+        sid[i * bm:(i + 1) * bm], eid[i] = sid[b * bm:(b + 1) * bm].clone(), live[b]
+    schedule = (sid, eid, torch.full_like(npp, 3 * bm))
+    dcase = to_device(case)
+    got = []
+    assert slices_launched(lambda: got.append(run_capi(case, bm, 64, 4, 3, dcase=dcase, schedule=schedule))) == slices
+    ref = orc.fused_moe_w8a8_up_down_oracle(case.x, case.x_scale, case.w, case.w_scale, case.w2, case.w2_scale, *schedule,
+                                            case.topk_weights, 8, bm, 1.5)
+    rows = sid[:3 * bm]
+    rows = torch.unique(rows[rows < m * 8] // 8).long()
+    check_close(got[0][rows], ref[rows], tag=f"k={k} slices={slices}")
+    assert int((got[0] != 0).any(1).sum()) == rows.numel()
