@@ -219,7 +219,7 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     // ====================================================================== control + gather warpgroups
     setmaxnreg_dec<40>();
     if (warp == W_MMA0 + 1) {
-        // (no role: one warp issues a chunk's four or eight UMMAs faster than they run)
+        // (no role: one warp issues a chunk's four or eight UMMAs faster than they run; setmaxnreg needs whole warpgroups)
     } else if (warp == W_MMA0) {
         // ------------------------------------------------------------------ UMMA issuer
         {
@@ -387,8 +387,9 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
         float fac[SPC];                      // s_h * topk weight * scaling per slice (reference :997-1003)
 
         const uint32_t tlane = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
-        // A wait that runs out does not leave the loops of the up phase: the abort flag lets every later wait return at once, and
-        // what was computed meanwhile is added nowhere (see in front of the down phase).
+        // A wait that runs out does not leave the loops of the up phase: with the abort flag raised every later wait returns after
+        // one batch of polls (0.3 ms, so 70 ms for four slices of 56 chunks), and what was computed meanwhile is added nowhere
+        // (see in front of the down phase).
         bool ok = true;
         uint32_t xph = 0;
         // ---- up-projection: promote each K chunk with its scales (reference :915-933).  The chunk loop is kept
