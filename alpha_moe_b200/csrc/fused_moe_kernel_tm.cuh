@@ -137,7 +137,8 @@ fused_moe_w8a8_up_down_sm100_tokmajor_kernel(const __grid_constant__ CUtensorMap
     // What the rest of the prologue depends on is requested together, before the set-up: the schedule's length, this block's
     // expert and the sorted ids this thread will need (a gather thread those of its rows, an epilogue thread its token's).
     constexpr int GROUPS = kTmRows / 4, MAXG = (GROUPS + kTmGatherWarps - 1) / kTmGatherWarps;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // (from lane 0: what depends on it is uniform in the warp for the compiler, too)
+    const int warp = __shfl_sync(0xFFFFFFFFu, static_cast<int>(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
     const int gather_warp = warp == W_G0 ? 0 : warp - W_G1 + 1;      // of the gather role only
     int pid_pre[MAXG];
     int expert;
