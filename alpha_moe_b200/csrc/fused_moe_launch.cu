@@ -183,9 +183,9 @@ int slices_per_cta(int K, int N, int block_m, int block_n, int stages, long long
 // Opts a kernel into the large dynamic shared-memory window once per device (atomically: several host threads
 // may launch at the same time).
 template <typename Kern>
-int ensure_smem_attr(Kern kern, std::atomic<int>* configured, int dev) {
+int ensure_smem_attr(Kern kern, std::atomic<int>* configured, int dev, int max_smem = kMaxDynSmem) {
     if (dev < kMaxDevices && configured[dev].load(std::memory_order_acquire)) return ALPHA_MOE_OK;
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
     if (dev < kMaxDevices) configured[dev].store(1, std::memory_order_release);
     return ALPHA_MOE_OK;
 }
@@ -219,11 +219,11 @@ int launch_dependent(Kern kern, int grid, int threads, int smem_bytes, int clust
     return ALPHA_MOE_OK;
 }
 
-template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false, bool GENERAL = false>
+template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false, bool GENERAL = false, bool DIRECT = false>
 int launch_variant(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
-    auto kern = amoe::fused_moe_w8a8_up_down_sm100_kernel<BMP, SPC, EW, PEERS, GENERAL>;
+    auto kern = amoe::fused_moe_w8a8_up_down_sm100_kernel<BMP, SPC, EW, PEERS, GENERAL, DIRECT>;
     static std::atomic<int> configured[kMaxDevices];
-    if (int rc = ensure_smem_attr(kern, configured, dev)) return rc;
+    if (int rc = ensure_smem_attr(kern, configured, dev, DIRECT ? kMaxDynSmem - amoe::kDirectSmem : kMaxDynSmem)) return rc;
     constexpr int threads = 128 * EW + 128;
     return launch_dependent(kern, grid, threads, smem_bytes, p.ksplit, stream, maps, p);
 }
@@ -649,11 +649,10 @@ tp_allreduce_kernel(TpExchange b, int nvec, int world, int rank, amoe::KernelSta
     }
 }
 
-int launch_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
-                 const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
-                 const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
-                 int M, int K, int N, int num_experts, int sorted_num, int block_m, int block_n, int warp_n, int stages,
-                 float scaling_factor, void* stream) {
+int check_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
+                const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
+                const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
+                int M, int K, int N, int num_experts, int sorted_num, int block_m, int block_n, int warp_n, int stages) {
     if (!x || !x_scale || !w || !w_scale || !w2 || !w2_scale || !outs || !sorted_token_ids || !expert_ids ||
         !num_tokens_post_padded || !topk_weights)
         return fail(ALPHA_MOE_E_ARG, "null pointer argument");
@@ -665,7 +664,6 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     if (tp_world > 1 && block_m > 64)
         return fail(ALPHA_MOE_E_ARG, "the fused tensor-parallel exchange serves small batches: block_m <= 64 (got %d); "
                                      "larger blocks run the plain operator followed by an all-reduce", block_m);
-    void* out = outs[tp_rank];
     if (M <= 0) return fail(ALPHA_MOE_E_ARG, "x must have at least one row (M=%d)", M);
     if (K <= 0 || K % 128 != 0) return fail(ALPHA_MOE_E_ARG, "K dimension must be a multiple of 128 (K=%d)", K);
     if (N <= 0 || N % 256 != 0) return fail(ALPHA_MOE_E_ARG, "N must be a multiple of 256 (N=%d)", N);
@@ -683,21 +681,44 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
         if (reinterpret_cast<uintptr_t>(outs[r]) & (token_major(block_m) ? 15 : 3))
             return fail(ALPHA_MOE_E_ARG, "out must be %d-byte aligned for block_m=%d", token_major(block_m) ? 16 : 4, block_m);
     if (static_cast<long long>(M) * top_k > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "M*top_k overflows int32");
+    return ALPHA_MOE_OK;
+}
 
+// What a launch uses.
+struct FusedPlan {
+    long long nblocks;       // schedule blocks that can be live at most
+    int spc, ksplit, depth, bmp, smem_bytes;
+};
+int plan_fused(const DeviceFacts& facts, int M, int top_k, int K, int N, int sorted_num, int block_m, int block_n, int stages,
+               FusedPlan* out) {
+    // Live blocks never exceed the number of assignments, so no more CTAs than that are launched.
+    out->nblocks = (static_cast<long long>(sorted_num) + block_m - 1) / block_m;
+    if (out->nblocks > static_cast<long long>(M) * top_k) out->nblocks = static_cast<long long>(M) * top_k;
+    const long long live_min = std::min(out->nblocks, (static_cast<long long>(M) * top_k + block_m - 1) / block_m);
+    out->spc = slices_per_cta(K, N, block_m, block_n, stages, live_min, facts.sms);
+    out->ksplit = choose_ksplit(block_m, out->spc, out->nblocks, N, K, stages, facts.clusters);
+    return plan(K, block_m, stages, out->spc, out->ksplit, &out->depth, &out->bmp, &out->smem_bytes);
+}
+
+// topk_ids: the batch's routing for a launch that takes it instead of a schedule (direct_schedule), else null.
+int launch_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
+                 const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
+                 const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
+                 int M, int K, int N, int num_experts, int sorted_num, int block_m, int block_n, int warp_n, int stages,
+                 float scaling_factor, void* stream, const int32_t* topk_ids = nullptr) {
+    if (int rc = check_fused(x, x_scale, w, w_scale, w2, w2_scale, outs, tp_world, tp_rank, sorted_token_ids, expert_ids,
+                             num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, sorted_num, block_m, block_n,
+                             warp_n, stages))
+        return rc;
+    void* out = outs[tp_rank];
     int dev = 0;
     CUDA_TRY(cudaGetDevice(&dev));
     DeviceFacts facts;
     if (int rc = device_facts(dev, &facts)) return rc;
-
-    // Live blocks never exceed the number of assignments, so no more CTAs than that are launched.
-    long long nblocks = (static_cast<long long>(sorted_num) + block_m - 1) / block_m;
-    if (nblocks > static_cast<long long>(M) * top_k) nblocks = static_cast<long long>(M) * top_k;
-    const long long live_min = std::min(nblocks, (static_cast<long long>(M) * top_k + block_m - 1) / block_m);
-    const int spc = slices_per_cta(K, N, block_m, block_n, stages, live_min, facts.sms);
-    const int ksplit = choose_ksplit(block_m, spc, nblocks, N, K, stages, facts.clusters);
-    int depth, bmp, smem_bytes;
-    if (int rc = plan(K, block_m, stages, spc, ksplit, &depth, &bmp, &smem_bytes)) return rc;
-
+    FusedPlan fp;
+    if (int rc = plan_fused(facts, M, top_k, K, N, sorted_num, block_m, block_n, stages, &fp)) return rc;
+    const int spc = fp.spc, ksplit = fp.ksplit, depth = fp.depth, bmp = fp.bmp, smem_bytes = fp.smem_bytes;
+    const long long nblocks = fp.nblocks;
     MapSet maps;
     if (int rc = get_maps(dev, w, w2, num_experts, N, K, &maps)) return rc;
 
@@ -713,6 +734,7 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     p.sorted_token_ids = sorted_token_ids;
     p.expert_ids = expert_ids;
     p.num_tokens_post_padded = num_tokens_post_padded;
+    p.topk_ids = topk_ids;
     p.topk_weights = topk_weights;
     p.top_k = top_k;
     p.M = M;
@@ -755,6 +777,7 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
             default: return launch_frag<64, 2, true>(maps, p, g, smem_bytes, dev, st);
         }
     }
+    if (topk_ids) return launch_variant<16, 1, 1, false, false, true>(maps, p, g, smem_bytes, dev, st);
     if (spc == 1) {
         switch (bmp) {
             case 16: return launch_variant<16, 1>(maps, p, g, smem_bytes, dev, st);
@@ -1001,6 +1024,26 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
     const long long numel = static_cast<long long>(M) * top_k;
     const long long sorted_num = numel + static_cast<long long>(num_experts) * (block_m - 1);
     if (sorted_num > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "schedule too long for int32");
+    void* outs[1] = {hidden_states};
+    bool direct = false;
+    if (numel <= amoe::kDirectMax && padded_block_m(block_m) == 16 && num_experts <= 1024 &&
+        check_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids, num_tokens_post_padded,
+                    topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num), block_m, block_n, warp_n,
+                    stages) == ALPHA_MOE_OK) {
+        int dev = 0;
+        DeviceFacts facts;
+        FusedPlan fp;
+        direct = cudaGetDevice(&dev) == cudaSuccess && device_facts(dev, &facts) == ALPHA_MOE_OK &&
+                 plan_fused(facts, M, top_k, K, N, static_cast<int>(sorted_num), block_m, block_n, stages, &fp) == ALPHA_MOE_OK &&
+                 fp.spc == 1 && fp.smem_bytes <= kMaxDynSmem - amoe::kDirectSmem;
+    }
+    if (direct) {
+        // A few tokens: the operator makes its schedule itself while the activations are quantised.
+        if (int rc = alpha_moe_b200_per_token_group_quant_fp8(hidden_states, x_fp8, x_scale, M, K, 1, stream)) return rc;
+        return launch_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids,
+                            num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num),
+                            block_m, block_n, warp_n, stages, scaling_factor, stream, topk_ids);
+    }
     // extra/sglang.patch:30-31: quantise, then clear the buffer the layer accumulates into; :33-35: the schedule
     // (one launch for both when the schedule fits one CTA)
     if (int rc = alpha_moe_b200_quant_and_align(hidden_states, x_fp8, x_scale, M, K, 1, topk_ids, top_k, num_experts,

@@ -251,3 +251,62 @@ def test_back_to_back_layers_with_changing_inputs_eager_and_from_a_graph():
             assert orc.rel_l2(hs.cpu(), ref) <= 2e-2, (rep, conf)
     from alpha_moe_b200 import capi
     assert capi.read_status(reset=True)[0] == 0
+
+
+@pytest.mark.parametrize("m,top_k,e,k,inter,bm,stages", [
+    (1, 1, 1, 128, 128, 16, 1),            # one assignment, one chunk, a ring of one slot
+    (1, 9, 24, 7168, 256, 16, 4),          # one token at the DeepSeek-V3 TP8 shard's sizes
+    (5, 9, 257, 1024, 256, 16, 2),
+    (3, 10, 512, 2048, 256, 16, 4),
+    (14, 9, 40, 384, 384, 8, 3),           # 126 assignments, several blocks of an expert, three slices
+    (16, 8, 1024, 256, 256, 8, 5),         # 128 assignments and 1024 experts, the most it takes
+    (43, 3, 16, 256, 256, 16, 3),          # 129 assignments: the schedule kernel again
+])
+@pytest.mark.parametrize("routing", ["topk", "duplicates", "outside", "none"])
+def test_small_batches_whose_operator_makes_its_own_schedule(m, top_k, e, k, inter, bm, stages, routing):
+    """Up to 128 assignments and blocks of up to 16 the layer call launches no schedule kernel: every CTA derives its block from
+    the routing.  Against the oracle on the reference's schedule, with experts chosen twice by a token, ids outside [0, E)
+    (ignored) and no valid id at all; eagerly and from a graph."""
+    from alpha_moe_b200 import capi
+    from alpha_moe_b200.layer import fused_experts_impl
+    g = torch.Generator().manual_seed(100 * m + top_k)
+    w, w_scale, w2, w2_scale = orc.make_weights(min(e, 24), k, inter, g)
+    if e > 24:                                             # few distinct experts, at both ends and in the middle of the range
+        pick = torch.arange(e) % 24
+        w, w2 = (t.view(torch.uint8)[pick].view(torch.float8_e4m3fn) for t in (w, w2))
+        w_scale, w2_scale = w_scale[pick], w2_scale[pick]
+    hidden = torch.randn(m, k, generator=g).to(torch.bfloat16)
+    ids = torch.stack([torch.randperm(e, generator=g)[:top_k] for _ in range(m)]).to(torch.int32)
+    if routing == "duplicates":
+        ids = torch.randint(max(0, e - 3), e, (m, top_k), generator=g, dtype=torch.int32)
+    elif routing == "outside":
+        ids[::2, ::2] = -1
+        ids[1::2, ::3] = e
+    elif routing == "none":
+        ids[:] = -7
+    wts = torch.rand(m, top_k, generator=g)
+    valid = (ids >= 0) & (ids < e)
+    xq, xs = orc.quant_token_groups(hidden)
+    sid, eid, npp = orc.moe_align_block_size(ids.clamp(0, e - 1), bm, e)      # (an ignored id is one of weight 0)
+    ref = orc.fused_moe_w8a8_up_down_oracle(xq, xs, w, w_scale, w2, w2_scale, sid, eid, npp, wts * valid, top_k, bm, 2.5)
+    args = [t.cuda() for t in (w, w_scale, w2, w2_scale, wts, ids)]
+    conf = {"block_m": bm, "block_n": 32, "warp_n": 8, "stages": stages}
+
+    def call(hs):
+        return fused_experts_impl(hs, *args, routed_scaling_factor=2.5, config=conf)
+
+    hs = hidden.cuda()
+    call(hs)
+    static = hidden.cuda()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(static)
+    for got in (hs, static):
+        if got is static:
+            graph.replay()
+        torch.cuda.synchronize()
+        assert capi.read_status(reset=True)[0] == 0
+        if not valid.any():
+            assert not got.any()
+        else:
+            assert orc.rel_l2(got.cpu(), ref) <= 2e-2
