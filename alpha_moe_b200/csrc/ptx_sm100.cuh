@@ -154,6 +154,11 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same without any ordering of memory accesses: at the end of a kernel, where no CTA may go while a peer still writes
+// into or reads from its shared memory.  (A releasing arrival would wait for the acknowledgement of all reductions.)
+__device__ __forceinline__ void cluster_sync_all_relaxed() {
+    asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 // shared::cta address -> address of the same location in the shared memory of CTA `rank` of the cluster
 __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
     uint32_t r;
@@ -162,6 +167,14 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t addr, uint32_t rank) {
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+// Two floats into a peer's shared memory, counted as 8 bytes by the peer's mbarrier (both addresses from mapa_shared): who has
+// waited for that barrier sees them.
+__device__ __forceinline__ void st_async_f32x2(uint32_t cluster_addr, float a, float b, uint32_t cluster_bar) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "r"(__float_as_uint(a)), "r"(__float_as_uint(b)));
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+                 ::"r"(cluster_addr), "l"(v), "r"(cluster_bar) : "memory");
 }
 __device__ __forceinline__ float ld_dsmem_f32(uint32_t cluster_addr) {
     float v;
