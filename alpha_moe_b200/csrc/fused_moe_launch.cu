@@ -700,7 +700,15 @@ int plan_fused(const DeviceFacts& facts, int M, int top_k, int K, int N, int sor
     return plan(K, block_m, stages, out->spc, out->ksplit, &out->depth, &out->bmp, &out->smem_bytes);
 }
 
-// topk_ids: the batch's routing for a launch that takes it instead of a schedule (direct_schedule), else null.
+// Whether there is room for what the DIRECT form adds: its words beside the ring (without costing a launch the second CTA of an
+// SM), and the histogram where the intermediate and the token scales go later.
+bool direct_fits(int K, int num_experts, const FusedPlan& fp) {
+    const int room = fp.smem_bytes <= kPairDynSmem ? kPairDynSmem : kMaxDynSmem;
+    return fp.smem_bytes + amoe::kDirectSmem <= room &&
+           amoe::direct_histogram_bytes(num_experts) <= fp.spc * 16 * 128 + K / 128 * 16 * 4;
+}
+
+// topk_ids: the batch's routing for a launch that takes it instead of a schedule, else null.
 int launch_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
                  const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
                  const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
@@ -777,7 +785,9 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
             default: return launch_frag<64, 2, true>(maps, p, g, smem_bytes, dev, st);
         }
     }
-    if (topk_ids) return launch_variant<16, 1, 1, false, false, true>(maps, p, g, smem_bytes, dev, st);
+    if (topk_ids)
+        return spc == 1 ? launch_variant<16, 1, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
+                        : launch_variant<16, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st);
     if (spc == 1) {
         switch (bmp) {
             case 16: return launch_variant<16, 1>(maps, p, g, smem_bytes, dev, st);
@@ -1035,10 +1045,10 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
         FusedPlan fp;
         direct = cudaGetDevice(&dev) == cudaSuccess && device_facts(dev, &facts) == ALPHA_MOE_OK &&
                  plan_fused(facts, M, top_k, K, N, static_cast<int>(sorted_num), block_m, block_n, stages, &fp) == ALPHA_MOE_OK &&
-                 fp.spc == 1 && fp.smem_bytes <= kMaxDynSmem - amoe::kDirectSmem;
+                 direct_fits(K, num_experts, fp);
     }
     if (direct) {
-        // A few tokens: the operator makes its schedule itself while the activations are quantised.
+        // Decode batches: the operator makes its schedule itself while the activations are quantised.
         if (int rc = alpha_moe_b200_per_token_group_quant_fp8(hidden_states, x_fp8, x_scale, M, K, 1, stream)) return rc;
         return launch_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids,
                             num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num),

@@ -258,13 +258,15 @@ def test_back_to_back_layers_with_changing_inputs_eager_and_from_a_graph():
     (1, 9, 24, 7168, 256, 16, 4),          # one token at the DeepSeek-V3 TP8 shard's sizes
     (5, 9, 257, 1024, 256, 16, 2),
     (3, 10, 512, 2048, 256, 16, 4),
-    (14, 9, 40, 384, 384, 8, 3),           # 126 assignments, several blocks of an expert, three slices
-    (16, 8, 1024, 256, 256, 8, 5),         # 128 assignments and 1024 experts, the most it takes
-    (43, 3, 16, 256, 256, 16, 3),          # 129 assignments: the schedule kernel again
+    (14, 9, 40, 384, 384, 8, 3),           # several blocks of an expert, three slices
+    (28, 9, 257, 512, 256, 8, 5),          # two slices per CTA (block_n = 64 from here on where even)
+    (57, 9, 257, 256, 512, 16, 3),         # 513 assignments: the third of a thread's eight
+    (256, 8, 1024, 256, 256, 8, 5),        # 2048 assignments and 1024 experts, the most it takes
+    (205, 10, 33, 128, 256, 16, 2),        # 2050 assignments: the schedule kernel again
 ])
 @pytest.mark.parametrize("routing", ["topk", "duplicates", "outside", "none"])
 def test_small_batches_whose_operator_makes_its_own_schedule(m, top_k, e, k, inter, bm, stages, routing):
-    """Up to 128 assignments and blocks of up to 16 the layer call launches no schedule kernel: every CTA derives its block from
+    """Up to 2048 assignments and blocks of up to 16 the layer call launches no schedule kernel: every CTA derives its block from
     the routing.  Against the oracle on the reference's schedule, with experts chosen twice by a token, ids outside [0, E)
     (ignored) and no valid id at all; eagerly and from a graph."""
     from alpha_moe_b200 import capi
@@ -290,7 +292,7 @@ def test_small_batches_whose_operator_makes_its_own_schedule(m, top_k, e, k, int
     sid, eid, npp = orc.moe_align_block_size(ids.clamp(0, e - 1), bm, e)      # (an ignored id is one of weight 0)
     ref = orc.fused_moe_w8a8_up_down_oracle(xq, xs, w, w_scale, w2, w2_scale, sid, eid, npp, wts * valid, top_k, bm, 2.5)
     args = [t.cuda() for t in (w, w_scale, w2, w2_scale, wts, ids)]
-    conf = {"block_m": bm, "block_n": 32, "warp_n": 8, "stages": stages}
+    conf = {"block_m": bm, "block_n": 32 if m < 28 else 64, "warp_n": 8 if m < 28 else 4, "stages": stages}
 
     def call(hs):
         return fused_experts_impl(hs, *args, routed_scaling_factor=2.5, config=conf)
