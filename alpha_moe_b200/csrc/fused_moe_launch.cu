@@ -183,9 +183,9 @@ int slices_per_cta(int K, int N, int block_m, int block_n, int stages, long long
 // Opts a kernel into the large dynamic shared-memory window once per device (atomically: several host threads
 // may launch at the same time).
 template <typename Kern>
-int ensure_smem_attr(Kern kern, std::atomic<int>* configured, int dev, int max_smem = kMaxDynSmem) {
+int ensure_smem_attr(Kern kern, std::atomic<int>* configured, int dev) {
     if (dev < kMaxDevices && configured[dev].load(std::memory_order_acquire)) return ALPHA_MOE_OK;
-    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, max_smem));
+    CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kMaxDynSmem));
     if (dev < kMaxDevices) configured[dev].store(1, std::memory_order_release);
     return ALPHA_MOE_OK;
 }
@@ -223,7 +223,7 @@ template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false, bo
 int launch_variant(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
     auto kern = amoe::fused_moe_w8a8_up_down_sm100_kernel<BMP, SPC, EW, PEERS, GENERAL, DIRECT>;
     static std::atomic<int> configured[kMaxDevices];
-    if (int rc = ensure_smem_attr(kern, configured, dev, DIRECT ? kMaxDynSmem - amoe::kDirectSmem : kMaxDynSmem)) return rc;
+    if (int rc = ensure_smem_attr(kern, configured, dev)) return rc;
     constexpr int threads = 128 * EW + 128;
     return launch_dependent(kern, grid, threads, smem_bytes, p.ksplit, stream, maps, p);
 }
@@ -700,12 +700,15 @@ int plan_fused(const DeviceFacts& facts, int M, int top_k, int K, int N, int sor
     return plan(K, block_m, stages, out->spc, out->ksplit, &out->depth, &out->bmp, &out->smem_bytes);
 }
 
-// Whether there is room for what the DIRECT form adds: its words beside the ring (without costing a launch the second CTA of an
-// SM), and the histogram where the intermediate and the token scales go later.
-bool direct_fits(int K, int num_experts, const FusedPlan& fp) {
-    const int room = fp.smem_bytes <= kPairDynSmem ? kPairDynSmem : kMaxDynSmem;
-    return fp.smem_bytes + amoe::kDirectSmem <= room &&
-           amoe::direct_histogram_bytes(num_experts) <= fp.spc * 16 * 128 + K / 128 * 16 * 4;
+// A 64-wide tile with a ring of at most two slots runs the single-warpgroup shape, two CTAs per SM
+// (227 KB per SM less 1 KB reserved per CTA leaves 113 KB of dynamic shared memory for each).
+bool pair64(const FusedPlan& fp) { return fp.bmp == 64 && fp.depth <= 2 && fp.smem_bytes <= kPairDynSmem; }
+
+// Whether the launch has a DIRECT form: the tiles of 16 tokens, and the wider ones with two slices where they have the fragment
+// epilogue's usual form and one epilogue warpgroup.
+bool has_direct_form(const FusedPlan& fp, long long numel, int num_experts) {
+    const bool shape = fp.bmp == 16 || (fp.spc == 2 && fp.depth >= 2 && (fp.bmp == 32 || pair64(fp)));
+    return shape && numel <= amoe::kDirectMax && amoe::direct_bytes(num_experts) <= fp.spc * fp.bmp * 128;
 }
 
 // topk_ids: the batch's routing for a launch that takes it instead of a schedule, else null.
@@ -764,9 +767,6 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     if (grid > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "grid too large");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int g = static_cast<int>(grid);
-    // A 64-wide tile with a ring of at most two slots runs the single-warpgroup shape, two CTAs per SM
-    // (227 KB per SM less 1 KB reserved per CTA leaves 113 KB of dynamic shared memory for each).
-    const bool pair64 = bmp == 64 && depth <= 2 && smem_bytes <= kPairDynSmem;
     if (token_major(block_m))
         return spc == 1 ? launch_tokmajor<1>(maps, p, g, smem_bytes, dev, st)
              : spc == 2 ? launch_tokmajor<2>(maps, p, g, smem_bytes, dev, st)
@@ -786,20 +786,22 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
         }
     }
     if (topk_ids)
-        return spc == 1 ? launch_variant<16, 1, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
-                        : launch_variant<16, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st);
+        return bmp == 32  ? launch_variant<32, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
+               : bmp == 64 ? launch_variant<64, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
+               : spc == 1  ? launch_variant<16, 1, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
+                           : launch_variant<16, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st);
     if (spc == 1) {
         switch (bmp) {
             case 16: return launch_variant<16, 1>(maps, p, g, smem_bytes, dev, st);
             case 32: return launch_variant<32, 1>(maps, p, g, smem_bytes, dev, st);
-            default: return pair64 ? launch_variant<64, 1, 1>(maps, p, g, smem_bytes, dev, st)
+            default: return pair64(fp) ? launch_variant<64, 1, 1>(maps, p, g, smem_bytes, dev, st)
                                    : launch_variant<64, 1>(maps, p, g, smem_bytes, dev, st);
         }
     }
     switch (bmp) {
         case 16: return launch_variant<16, 2>(maps, p, g, smem_bytes, dev, st);
         case 32: return launch_frag<32, 1, false>(maps, p, g, smem_bytes, dev, st);
-        default: return pair64 ? launch_frag<64, 1, false>(maps, p, g, smem_bytes, dev, st)
+        default: return pair64(fp) ? launch_frag<64, 1, false>(maps, p, g, smem_bytes, dev, st)
                                : launch_frag<64, 2, false>(maps, p, g, smem_bytes, dev, st);
     }
 }
@@ -1036,7 +1038,7 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
     if (sorted_num > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "schedule too long for int32");
     void* outs[1] = {hidden_states};
     bool direct = false;
-    if (numel <= amoe::kDirectMax && padded_block_m(block_m) == 16 && num_experts <= 1024 &&
+    if (numel <= amoe::kDirectMax && num_experts <= 1024 &&
         check_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids, num_tokens_post_padded,
                     topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num), block_m, block_n, warp_n,
                     stages) == ALPHA_MOE_OK) {
@@ -1045,7 +1047,7 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
         FusedPlan fp;
         direct = cudaGetDevice(&dev) == cudaSuccess && device_facts(dev, &facts) == ALPHA_MOE_OK &&
                  plan_fused(facts, M, top_k, K, N, static_cast<int>(sorted_num), block_m, block_n, stages, &fp) == ALPHA_MOE_OK &&
-                 direct_fits(K, num_experts, fp);
+                 has_direct_form(fp, numel, num_experts);
     }
     if (direct) {
         // Decode batches: the operator makes its schedule itself while the activations are quantised.

@@ -261,12 +261,16 @@ def test_back_to_back_layers_with_changing_inputs_eager_and_from_a_graph():
     (14, 9, 40, 384, 384, 8, 3),           # several blocks of an expert, three slices
     (28, 9, 257, 512, 256, 8, 5),          # two slices per CTA (block_n = 64 from here on where even)
     (57, 9, 257, 256, 512, 16, 3),         # 513 assignments: the third of a thread's eight
-    (256, 8, 1024, 256, 256, 8, 5),        # 2048 assignments and 1024 experts, the most it takes
-    (205, 10, 33, 128, 256, 16, 2),        # 2050 assignments: the schedule kernel again
+    (256, 8, 1024, 256, 256, 8, 5),        # 2048 assignments, the last that a thread reads once; 1024 experts
+    (205, 10, 33, 128, 256, 16, 2),        # 2050: ids read twice
+    (205, 10, 300, 128, 256, 32, 2),       # tiles of 32 and 64 tokens
+    (33, 9, 1024, 256, 512, 64, 2),
+    (819, 10, 50, 128, 256, 48, 2),        # 8190 assignments, the last of a thread's 32
+    (820, 10, 50, 128, 256, 64, 2),        # 8200: the schedule kernel again
 ])
 @pytest.mark.parametrize("routing", ["topk", "duplicates", "outside", "none"])
 def test_small_batches_whose_operator_makes_its_own_schedule(m, top_k, e, k, inter, bm, stages, routing):
-    """Up to 2048 assignments and blocks of up to 16 the layer call launches no schedule kernel: every CTA derives its block from
+    """Up to 8192 assignments in blocks of up to 64 the layer call launches no schedule kernel: every CTA derives its block from
     the routing.  Against the oracle on the reference's schedule, with experts chosen twice by a token, ids outside [0, E)
     (ignored) and no valid id at all; eagerly and from a graph."""
     from alpha_moe_b200 import capi
