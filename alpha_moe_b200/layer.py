@@ -1,32 +1,25 @@
 """The body the reference's serving patch gives `fused_experts_impl` (extra/sglang.patch:25-40), on this
 library's own kernels: knob look-up for the batch size, activation quantisation, clearing of the buffer the
 layer accumulates into, block schedule, fused operator.  `hidden_states` holds the layer output on return,
-as in the patch.  Buffers come from torch; the work is one C-ABI call."""
+as in the patch.  Checks, buffers and the C-ABI call are one torch operator."""
 from __future__ import annotations
 
-import contextlib
 import os
 
 import torch
 
-from . import capi
+from . import capi, load_torch_op
 from .utils import get_best_config
 
-try:        # the raw handle without a Stream object around it (one microsecond of an eager call's host time)
-    from torch._C import _cuda_getCurrentRawStream as _current_stream
-except ImportError:
-    def _current_stream(device_index: int) -> int:
-        return torch.cuda.current_stream(device_index).cuda_stream
-
-
-def _up(n: int) -> int:
-    return (n + 255) & ~255
+load_torch_op()
+_fused_experts = torch.ops.alpha_moe._fused_experts.default
 
 
 def _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids) -> None:
     """The checks the torch operator makes on its tensors (csrc/torch_interface.cpp:58-76 of the reference, plus
     the dtype / device / shape checks this library's operator adds), made here before any raw pointer is taken:
-    this path goes straight to the C ABI, which sees only addresses."""
+    this path goes straight to the C ABI, which sees only addresses.  (CUDA tensors are checked by the same rules in
+    csrc/torch_interface.cpp.)"""
     # (written out: messages are only put together for a call that fails)
     if hidden_states.dtype != torch.bfloat16 or hidden_states.dim() != 2 or not hidden_states.is_contiguous():
         raise RuntimeError("hidden_states must be a contiguous 2-D bfloat16 tensor")
@@ -74,44 +67,18 @@ def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: 
     topk_weights f32 [M,top_k].  `config`: a knob dict, a table path, or None for $ALPHA_MOE_CONFIG."""
     if tuple(block_shape) != (128, 128):
         raise ValueError("only 128 x 128 block scales are supported (the operator's scale layout)")
-    _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids)
     if not hidden_states.is_cuda:
+        _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids)
         raise RuntimeError("hidden_states must be a CUDA tensor (there is no CPU implementation)")
-    m, k = hidden_states.shape
-    e, n, _ = w1.shape
-    top_k = topk_ids.shape[1]
     if isinstance(config, dict):
         conf = config
     else:
         path = config or os.getenv("ALPHA_MOE_CONFIG")
         if not path:
             raise RuntimeError("no knob table: pass config= or set ALPHA_MOE_CONFIG")
-        conf = get_best_config(path, m)
-    block_m, bn, wn, stages = conf["block_m"], conf["block_n"], conf["warp_n"], conf["stages"]
-    dev = hidden_states.device
-    ids = topk_ids if topk_ids.dtype == torch.int32 and topk_ids.is_contiguous() else topk_ids.to(torch.int32).contiguous()
-    wts = (topk_weights if topk_weights.dtype == torch.float32 and topk_weights.is_contiguous()
-           else topk_weights.to(torch.float32).contiguous())
-    # One allocation holds every intermediate buffer (256-byte aligned pieces); at one token the call is bound by its
-    # host time, and seven allocations were a third of it.
-    numel = m * top_k
-    total = numel + e * (block_m - 1)
-    ws_bytes = capi.align_workspace_bytes(numel, e)
-    x_s = _up(m * k)
-    sorted_ids = x_s + _up(m * (k // 128) * 4)
-    expert_ids = sorted_ids + _up(total * 4)
-    num_post_pad = expert_ids + _up((total + block_m - 1) // block_m * 4)
-    ws = num_post_pad + 256
-    buf = torch.empty(ws + ws_bytes, dtype=torch.uint8, device=dev)
-    base = buf.data_ptr()
-    if dev.index == torch.cuda.current_device():
-        on_device = contextlib.nullcontext()
-    else:
-        on_device = torch.cuda.device(dev)
-    with on_device:
-        capi.fused_experts(hidden_states.data_ptr(), base, base + x_s, w1.data_ptr(), w1_scale.data_ptr(),
-                           w2.data_ptr(), w2_scale.data_ptr(), ids.data_ptr(), wts.data_ptr(), top_k, m, k, n, e,
-                           base + sorted_ids, base + expert_ids, base + num_post_pad, base + ws if ws_bytes else 0,
-                           block_m, bn, wn, stages, float(routed_scaling_factor or 1.0),
-                           _current_stream(dev.index))
+        conf = get_best_config(path, hidden_states.size(0))
+    rc = _fused_experts(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, conf["block_m"], conf["block_n"],
+                        conf["warp_n"], conf["stages"], float(routed_scaling_factor or 1.0))
+    if rc != 0:
+        capi._check(rc)
     return hidden_states

@@ -316,3 +316,55 @@ def test_small_batches_whose_operator_makes_its_own_schedule(m, top_k, e, k, int
             assert not got.any()
         else:
             assert orc.rel_l2(got.cpu(), ref) <= 2e-2
+
+
+def test_layer_call_refuses_cuda_tensors_in_the_words_of_the_host_checks():
+    """fused_experts_impl checks CUDA tensors inside its operator: what _check_layer_arguments refuses is refused with the same
+    message, an ABI error keeps its type, and the buffer is left alone."""
+    from alpha_moe_b200 import capi
+    from alpha_moe_b200.layer import _check_layer_arguments, fused_experts_impl
+    e, n, k, m, top_k = 4, 256, 256, 3, 2
+    f8 = torch.float8_e4m3fn
+    good = dict(
+        hidden_states=torch.ones(m, k, dtype=torch.bfloat16, device="cuda", requires_grad=True),
+        w1=torch.zeros(e, n, k, dtype=f8, device="cuda"), w1_scale=torch.zeros(e, n // 128, k // 128, device="cuda"),
+        w2=torch.zeros(e, k, n // 2, dtype=f8, device="cuda"), w2_scale=torch.zeros(e, k // 128, n // 256, device="cuda"),
+        topk_weights=torch.zeros(m, top_k, device="cuda"), topk_ids=torch.zeros(m, top_k, dtype=torch.int32, device="cuda"))
+    conf = dict(block_m=16, block_n=32, warp_n=8, stages=3)
+
+    def call(knobs=conf, **change):
+        a = dict(good, **change)
+        return fused_experts_impl(a["hidden_states"], a["w1"], a["w1_scale"], a["w2"], a["w2_scale"], a["topk_weights"],
+                                  a["topk_ids"], config=knobs)
+
+    bad = [
+        dict(hidden_states=torch.zeros(m, k, device="cuda")),
+        dict(hidden_states=torch.zeros(m, 2 * k, dtype=torch.bfloat16, device="cuda")[:, ::2]),
+        dict(hidden_states=torch.zeros(0, k, dtype=torch.bfloat16, device="cuda")),
+        dict(w1=torch.zeros(e, n, k // 2, dtype=f8, device="cuda")),
+        dict(w1=torch.zeros(e, 2 * n, k, dtype=f8, device="cuda")[:, ::2]),
+        dict(w2=torch.zeros(e, k, n, dtype=f8, device="cuda")),
+        dict(w2=torch.zeros(e, k, n // 2, dtype=torch.uint8, device="cuda")),
+        dict(w1_scale=torch.zeros(e, n // 128, k // 128 + 1, device="cuda")),
+        dict(w2_scale=torch.zeros(e, k // 128, n // 256, dtype=torch.float64, device="cuda")),
+        dict(w2_scale=torch.zeros(e, k // 128, n // 256)),
+        dict(topk_ids=torch.zeros(m + 1, top_k, dtype=torch.int32, device="cuda")),
+        dict(topk_weights=torch.zeros(m, top_k + 1, device="cuda")),
+    ]
+    for change in bad:
+        with pytest.raises(RuntimeError) as want:
+            _check_layer_arguments(**dict(good, **change))
+        with pytest.raises(RuntimeError) as got:
+            call(**change)
+        assert str(want.value) in str(got.value), (change, str(got.value))
+    for knobs in (dict(conf, block_m=0), dict(conf, stages=9), dict(conf, block_m=136)):
+        with pytest.raises(RuntimeError):
+            call(knobs)
+    with pytest.raises(capi.AlphaMoeError, match="stages"):
+        call(dict(conf, stages=9, block_m=128, block_n=64, warp_n=4))
+    torch.cuda.synchronize()
+    good["hidden_states"].data.fill_(1)
+    # other dtypes and layouts of the routing are converted; a buffer that requires gradients is overwritten all the same
+    out = call(topk_ids=torch.zeros(top_k, m, dtype=torch.int64, device="cuda").t(),
+               topk_weights=torch.zeros(m, top_k, dtype=torch.float64, device="cuda"))
+    assert out is good["hidden_states"] and not out.detach().any() and out.grad_fn is None
