@@ -15,6 +15,12 @@ load_torch_op()
 _fused_experts = torch.ops.alpha_moe._fused_experts.default
 
 
+@torch.compiler.disable
+def _fused_experts_outside_graphs(*args) -> int:
+    """For torch.compile: the call (in place, an error code back) stays outside its graphs."""
+    return _fused_experts(*args)
+
+
 def _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids) -> None:
     """The checks the torch operator makes on its tensors (csrc/torch_interface.cpp:58-76 of the reference, plus
     the dtype / device / shape checks this library's operator adds), made here before any raw pointer is taken:
@@ -77,8 +83,9 @@ def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: 
         if not path:
             raise RuntimeError("no knob table: pass config= or set ALPHA_MOE_CONFIG")
         conf = get_best_config(path, hidden_states.size(0))
-    rc = _fused_experts(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, conf["block_m"], conf["block_n"],
-                        conf["warp_n"], conf["stages"], float(routed_scaling_factor or 1.0))
+    call = _fused_experts_outside_graphs if torch.compiler.is_compiling() else _fused_experts
+    rc = call(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, conf["block_m"], conf["block_n"],
+              conf["warp_n"], conf["stages"], float(routed_scaling_factor or 1.0))
     if rc != 0:
         capi._check(rc)
     return hidden_states

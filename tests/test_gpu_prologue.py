@@ -368,3 +368,25 @@ def test_layer_call_refuses_cuda_tensors_in_the_words_of_the_host_checks():
     out = call(topk_ids=torch.zeros(top_k, m, dtype=torch.int64, device="cuda").t(),
                topk_weights=torch.zeros(m, top_k, dtype=torch.float64, device="cuda"))
     assert out is good["hidden_states"] and not out.detach().any() and out.grad_fn is None
+
+
+@pytest.mark.parametrize("backend", ["eager", "aot_eager"])
+def test_layer_call_inside_a_compiled_function(backend):
+    """torch.compile breaks its graph at the layer call, as it did when the call went through ctypes."""
+    from alpha_moe_b200.layer import fused_experts_impl
+    e, k, inter, m, top_k = 8, 256, 256, 5, 2
+    g = torch.Generator().manual_seed(9)
+    dw = [t.cuda() for t in orc.make_weights(e, k, inter, g)]
+    x = torch.randn(m, k, generator=g).to(torch.bfloat16).cuda()
+    ids, wts = orc.route_topk(torch.randn(m, e, generator=g), top_k)
+    ids, wts = ids.cuda(), wts.cuda()
+    conf = dict(block_m=16, block_n=32, warp_n=8, stages=3)
+
+    def layer(h):
+        return fused_experts_impl(h, *dw, wts, ids, routed_scaling_factor=2.5, config=conf) * 2
+
+    want = layer(x.clone())
+    torch._dynamo.reset()
+    h = x.clone()
+    got = torch.compile(layer, backend=backend)(h)
+    assert orc.rel_l2(got.cpu(), want.cpu()) <= 1e-2 and orc.rel_l2(2 * h.cpu(), want.cpu()) <= 1e-2
