@@ -711,41 +711,42 @@ bool has_direct_form(const FusedPlan& fp, long long numel, int num_experts) {
     return shape && numel <= amoe::kDirectMax && amoe::direct_bytes(num_experts) <= fp.spc * fp.bmp * 128;
 }
 
-// topk_ids: the batch's routing for a launch that takes it instead of a schedule, else null.
-int launch_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
-                 const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
-                 const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
-                 int M, int K, int N, int num_experts, int sorted_num, int block_m, int block_n, int warp_n, int stages,
-                 float scaling_factor, void* stream, const int32_t* topk_ids = nullptr) {
+// One launch of the operator, checked and planned: nothing but a CUDA error can refuse it any more.
+struct FusedLaunch {
+    MapSet maps;
+    amoe::MoeParams p;
+    FusedPlan plan;
+    int grid, dev;
+};
+int prepare_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
+                  const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
+                  const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
+                  int M, int K, int N, int num_experts, int sorted_num, int block_m, int block_n, int warp_n, int stages,
+                  float scaling_factor, FusedLaunch* fl) {
     if (int rc = check_fused(x, x_scale, w, w_scale, w2, w2_scale, outs, tp_world, tp_rank, sorted_token_ids, expert_ids,
                              num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, sorted_num, block_m, block_n,
                              warp_n, stages))
         return rc;
-    void* out = outs[tp_rank];
-    int dev = 0;
-    CUDA_TRY(cudaGetDevice(&dev));
+    CUDA_TRY(cudaGetDevice(&fl->dev));
     DeviceFacts facts;
-    if (int rc = device_facts(dev, &facts)) return rc;
-    FusedPlan fp;
+    if (int rc = device_facts(fl->dev, &facts)) return rc;
+    FusedPlan& fp = fl->plan;
     if (int rc = plan_fused(facts, M, top_k, K, N, sorted_num, block_m, block_n, stages, &fp)) return rc;
-    const int spc = fp.spc, ksplit = fp.ksplit, depth = fp.depth, bmp = fp.bmp, smem_bytes = fp.smem_bytes;
-    const long long nblocks = fp.nblocks;
-    MapSet maps;
-    if (int rc = get_maps(dev, w, w2, num_experts, N, K, &maps)) return rc;
+    if (int rc = get_maps(fl->dev, w, w2, num_experts, N, K, &fl->maps)) return rc;
 
-    amoe::MoeParams p;
+    amoe::MoeParams& p = fl->p;
     p.x = static_cast<const uint8_t*>(x);
     p.x_scale = x_scale;
     p.w_scale = w_scale;
     p.w2_scale = w2_scale;
-    p.out = static_cast<__nv_bfloat16*>(out);
+    p.out = static_cast<__nv_bfloat16*>(outs[tp_rank]);
     p.tp_world = tp_world;
     for (int i = 0; i < amoe::kMaxTpWorld - 1; ++i)       // the peers, starting behind this rank so that traffic spreads
         p.out_more[i] = i + 1 < tp_world ? static_cast<__nv_bfloat16*>(outs[(tp_rank + 1 + i) % tp_world]) : nullptr;
     p.sorted_token_ids = sorted_token_ids;
     p.expert_ids = expert_ids;
     p.num_tokens_post_padded = num_tokens_post_padded;
-    p.topk_ids = topk_ids;
+    p.topk_ids = nullptr;
     p.topk_weights = topk_weights;
     p.top_k = top_k;
     p.M = M;
@@ -754,8 +755,8 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     p.E = num_experts;
     p.sorted_num = sorted_num;
     p.block_m = block_m;
-    p.stages = depth;
-    p.ksplit = ksplit;
+    p.stages = fp.depth;
+    p.ksplit = fp.ksplit;
     p.scaling = scaling_factor;
     p.out_vec16 = 1;
     for (int r = 0; r < tp_world; ++r)
@@ -763,15 +764,25 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
     p.xs_vec4 = (K / 128) % 4 == 0 && (reinterpret_cast<uintptr_t>(x_scale) & 15) == 0;
     p.status = facts.status;
 
-    const long long grid = nblocks * (N / 256 / spc) * ksplit;
+    const long long grid = fp.nblocks * (N / 256 / fp.spc) * fp.ksplit;
     if (grid > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "grid too large");
+    fl->grid = static_cast<int>(grid);
+    return ALPHA_MOE_OK;
+}
+
+// topk_ids: the batch's routing for a launch that takes it instead of a schedule (has_direct_form), else null.
+int launch_prepared(FusedLaunch& fl, void* stream, const int32_t* topk_ids = nullptr) {
+    fl.p.topk_ids = topk_ids;
+    const MapSet& maps = fl.maps;
+    const amoe::MoeParams& p = fl.p;
+    const FusedPlan& fp = fl.plan;
+    const int spc = fp.spc, bmp = fp.bmp, smem_bytes = fp.smem_bytes, dev = fl.dev, g = fl.grid;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    const int g = static_cast<int>(grid);
-    if (token_major(block_m))
+    if (token_major(p.block_m))
         return spc == 1 ? launch_tokmajor<1>(maps, p, g, smem_bytes, dev, st)
              : spc == 2 ? launch_tokmajor<2>(maps, p, g, smem_bytes, dev, st)
                         : launch_tokmajor<4>(maps, p, g, smem_bytes, dev, st);
-    if (tp_world > 1) {       // the form that adds into the peers' buffers: one shape per tile width
+    if (p.tp_world > 1) {       // the form that adds into the peers' buffers: one shape per tile width
         if (spc == 1) {
             switch (bmp) {
                 case 16: return launch_variant<16, 1, 1, true>(maps, p, g, smem_bytes, dev, st);
@@ -804,6 +815,19 @@ int launch_fused(const void* x, const float* x_scale, const void* w, const float
         default: return pair64(fp) ? launch_frag<64, 1, false>(maps, p, g, smem_bytes, dev, st)
                                : launch_frag<64, 2, false>(maps, p, g, smem_bytes, dev, st);
     }
+}
+
+int launch_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
+                 const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
+                 const int32_t* expert_ids, const int32_t* num_tokens_post_padded, const float* topk_weights, int top_k,
+                 int M, int K, int N, int num_experts, int sorted_num, int block_m, int block_n, int warp_n, int stages,
+                 float scaling_factor, void* stream) {
+    FusedLaunch fl;
+    if (int rc = prepare_fused(x, x_scale, w, w_scale, w2, w2_scale, outs, tp_world, tp_rank, sorted_token_ids, expert_ids,
+                               num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, sorted_num, block_m, block_n,
+                               warp_n, stages, scaling_factor, &fl))
+        return rc;
+    return launch_prepared(fl, stream);
 }
 
 }  // namespace
@@ -1036,25 +1060,18 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
     const long long numel = static_cast<long long>(M) * top_k;
     const long long sorted_num = numel + static_cast<long long>(num_experts) * (block_m - 1);
     if (sorted_num > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "schedule too long for int32");
+    // Everything that can refuse the operator is settled before the quantiser clears hidden_states: a refused call leaves the
+    // caller's activations alone.
     void* outs[1] = {hidden_states};
-    bool direct = false;
-    if (numel <= amoe::kDirectMax && num_experts <= 1024 &&
-        check_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids, num_tokens_post_padded,
-                    topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num), block_m, block_n, warp_n,
-                    stages) == ALPHA_MOE_OK) {
-        int dev = 0;
-        DeviceFacts facts;
-        FusedPlan fp;
-        direct = cudaGetDevice(&dev) == cudaSuccess && device_facts(dev, &facts) == ALPHA_MOE_OK &&
-                 plan_fused(facts, M, top_k, K, N, static_cast<int>(sorted_num), block_m, block_n, stages, &fp) == ALPHA_MOE_OK &&
-                 has_direct_form(fp, numel, num_experts);
-    }
-    if (direct) {
+    FusedLaunch fl;
+    if (int rc = prepare_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids,
+                               num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num),
+                               block_m, block_n, warp_n, stages, scaling_factor, &fl))
+        return rc;
+    if (num_experts <= 1024 && has_direct_form(fl.plan, numel, num_experts)) {
         // Decode batches: the operator makes its schedule itself while the activations are quantised.
         if (int rc = alpha_moe_b200_per_token_group_quant_fp8(hidden_states, x_fp8, x_scale, M, K, 1, stream)) return rc;
-        return launch_fused(x_fp8, x_scale, w, w_scale, w2, w2_scale, outs, 1, 0, sorted_token_ids, expert_ids,
-                            num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num),
-                            block_m, block_n, warp_n, stages, scaling_factor, stream, topk_ids);
+        return launch_prepared(fl, stream, topk_ids);
     }
     // extra/sglang.patch:30-31: quantise, then clear the buffer the layer accumulates into; :33-35: the schedule
     // (one launch for both when the schedule fits one CTA)
@@ -1062,11 +1079,7 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
                                                 block_m, sorted_token_ids, expert_ids, num_tokens_post_padded,
                                                 align_workspace, stream))
         return rc;
-    // :38-40
-    return alpha_moe_b200_fused_moe_w8a8_up_down(x_fp8, x_scale, w, w_scale, w2, w2_scale, hidden_states, sorted_token_ids,
-                                                 expert_ids, num_tokens_post_padded, topk_weights, top_k, M, K, N,
-                                                 num_experts, static_cast<int>(sorted_num), block_m, block_n, warp_n,
-                                                 stages, scaling_factor, stream);
+    return launch_prepared(fl, stream);      // :38-40
 }
 
 

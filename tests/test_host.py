@@ -90,7 +90,8 @@ def test_capi_rejects_bad_arguments_without_a_gpu():
 
 
 def test_fused_experts_entry_rejects_bad_arguments_without_a_gpu():
-    """The single-call layer entry validates before it enqueues anything."""
+    """The single-call layer entry validates before it enqueues anything: what only the operator refuses, too, because the
+    quantiser in front of it clears hidden_states."""
     from alpha_moe_b200 import capi
     p = 0x1000
     base = dict(hidden_states=p, x_fp8=p, x_scale=p, w=p, w_scale=p, w2=p, w2_scale=p, topk_ids=p, topk_weights=p,
@@ -101,6 +102,14 @@ def test_fused_experts_entry_rejects_bad_arguments_without_a_gpu():
                      (dict(block_m=12), "block_m"), (dict(block_m=200), "block_m"), (dict(K=500), "multiple of 128")):
         with pytest.raises(capi.AlphaMoeError, match=msg):
             capi.fused_experts(*dict(base, **bad).values())
+    # batches whose operator makes its own schedule, whose schedule rides with the quantiser, and that run beside it
+    for batch in (dict(), dict(block_m=128), dict(M=4096), dict(M=4096, block_m=128)):
+        for bad, msg in ((dict(stages=9), "stages"), (dict(stages=0), "stages"), (dict(block_n=64), "block_n"),
+                         (dict(warp_n=4), "block_n"), (dict(w=p + 8), "aligned"), (dict(w2=p + 8), "aligned"),
+                         (dict(x_fp8=p + 8), "aligned"), (dict(topk_weights=0), "null"), (dict(w_scale=0), "null"),
+                         (dict(N=384), "multiple of 256")):
+            with pytest.raises(capi.AlphaMoeError, match=msg):
+                capi.fused_experts(*dict(base, **batch, **bad).values())
 
 
 def test_plan_fits_shared_memory_for_every_knob():
