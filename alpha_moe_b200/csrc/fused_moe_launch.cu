@@ -1060,6 +1060,9 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
     const long long numel = static_cast<long long>(M) * top_k;
     const long long sorted_num = numel + static_cast<long long>(num_experts) * (block_m - 1);
     if (sorted_num > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "schedule too long for int32");
+    // (asked for whether or not this launch builds its schedule there: which form it takes is not the caller's to know)
+    if (!align_workspace && alpha_moe_b200_align_workspace_bytes(static_cast<int>(numel), num_experts) > 0)
+        return fail(ALPHA_MOE_E_ARG, "align_workspace is required for %lld assignments", numel);
     // Everything that can refuse the operator is settled before the quantiser clears hidden_states: a refused call leaves the
     // caller's activations alone.
     void* outs[1] = {hidden_states};

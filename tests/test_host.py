@@ -103,13 +103,17 @@ def test_fused_experts_entry_rejects_bad_arguments_without_a_gpu():
         with pytest.raises(capi.AlphaMoeError, match=msg):
             capi.fused_experts(*dict(base, **bad).values())
     # batches whose operator makes its own schedule, whose schedule rides with the quantiser, and that run beside it
-    for batch in (dict(), dict(block_m=128), dict(M=4096), dict(M=4096, block_m=128)):
+    for batch in (dict(), dict(block_m=128), dict(M=4096, align_workspace=p), dict(M=4096, align_workspace=p, block_m=128)):
         for bad, msg in ((dict(stages=9), "stages"), (dict(stages=0), "stages"), (dict(block_n=64), "block_n"),
                          (dict(warp_n=4), "block_n"), (dict(w=p + 8), "aligned"), (dict(w2=p + 8), "aligned"),
                          (dict(x_fp8=p + 8), "aligned"), (dict(topk_weights=0), "null"), (dict(w_scale=0), "null"),
                          (dict(N=384), "multiple of 256")):
             with pytest.raises(capi.AlphaMoeError, match=msg):
                 capi.fused_experts(*dict(base, **batch, **bad).values())
+    # scratch for the schedule's histogram: needed above 1024 assignments, also by batches whose operator makes its own schedule
+    for m in (513, 900, 4096, 4097):
+        with pytest.raises(capi.AlphaMoeError, match="workspace"):
+            capi.fused_experts(*dict(base, M=m).values())
 
 
 def test_plan_fits_shared_memory_for_every_knob():
