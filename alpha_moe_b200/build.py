@@ -51,7 +51,7 @@ def _cuda_home() -> str:
 def build_capi(force: bool = False, verbose: bool = False) -> str:
     srcs = [os.path.join(CSRC, s) for s in CUDA_SOURCES if os.path.exists(os.path.join(CSRC, s))]
     deps = srcs + [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".cuh")]
-    deps.append(os.path.join(HERE, "..", "include", "alpha_moe_b200.h"))
+    deps += [os.path.join(CSRC, "capi_internal.h"), os.path.join(HERE, "..", "include", "alpha_moe_b200.h")]
     if not force and _newer(CAPI_LIB, deps):
         return CAPI_LIB
     nvcc = os.path.join(_cuda_home(), "bin", "nvcc")
@@ -68,7 +68,7 @@ def build_torch_op(force: bool = False) -> str:
     from torch.utils import cpp_extension
 
     src = os.path.join(CSRC, "torch_interface.cpp")
-    deps = [src, os.path.join(HERE, "..", "include", "alpha_moe_b200.h")]
+    deps = [src, os.path.join(CSRC, "capi_internal.h"), os.path.join(HERE, "..", "include", "alpha_moe_b200.h")]
     if not force and _newer(TORCH_LIB, deps) and _newer(TORCH_LIB, [CAPI_LIB]):
         return TORCH_LIB
     torch_lib = os.path.join(os.path.dirname(torch.__file__), "lib")

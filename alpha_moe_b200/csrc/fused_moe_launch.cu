@@ -219,7 +219,7 @@ int launch_dependent(Kern kern, int grid, int threads, int smem_bytes, int clust
     return ALPHA_MOE_OK;
 }
 
-template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false, bool GENERAL = false, bool DIRECT = false>
+template <int BMP, int SPC, int EW = (BMP >= 64 ? 2 : 1), bool PEERS = false, bool GENERAL = false, int DIRECT = 0>
 int launch_variant(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
     auto kern = amoe::fused_moe_w8a8_up_down_sm100_kernel<BMP, SPC, EW, PEERS, GENERAL, DIRECT>;
     static std::atomic<int> configured[kMaxDevices];
@@ -234,6 +234,16 @@ template <int BMP, int EW, bool PEERS>
 int launch_frag(const MapSet& maps, const amoe::MoeParams& p, int grid, int smem_bytes, int dev, cudaStream_t stream) {
     return p.stages == 1 || !p.out_vec16 ? launch_variant<BMP, 2, EW, PEERS, true>(maps, p, grid, smem_bytes, dev, stream)
                                           : launch_variant<BMP, 2, EW, PEERS, false>(maps, p, grid, smem_bytes, dev, stream);
+}
+
+// The forms that make their schedule themselves (has_direct_form).
+template <int DIRECT>
+int launch_direct(const MapSet& maps, const amoe::MoeParams& p, int bmp, int spc, int grid, int smem_bytes, int dev,
+                  cudaStream_t stream) {
+    return bmp == 32  ? launch_variant<32, 2, 1, false, false, DIRECT>(maps, p, grid, smem_bytes, dev, stream)
+           : bmp == 64 ? launch_variant<64, 2, 1, false, false, DIRECT>(maps, p, grid, smem_bytes, dev, stream)
+           : spc == 1  ? launch_variant<16, 1, 1, false, false, DIRECT>(maps, p, grid, smem_bytes, dev, stream)
+                       : launch_variant<16, 2, 1, false, false, DIRECT>(maps, p, grid, smem_bytes, dev, stream);
 }
 
 template <int SPC>
@@ -770,8 +780,9 @@ int prepare_fused(const void* x, const float* x_scale, const void* w, const floa
     return ALPHA_MOE_OK;
 }
 
-// topk_ids: the batch's routing for a launch that takes it instead of a schedule (has_direct_form), else null.
-int launch_prepared(FusedLaunch& fl, void* stream, const int32_t* topk_ids = nullptr) {
+// topk_ids: the batch's routing for a launch that takes it instead of a schedule (has_direct_form), else null; write_schedule: such
+// a launch fills the schedule's buffers, too.
+int launch_prepared(FusedLaunch& fl, void* stream, const int32_t* topk_ids = nullptr, bool write_schedule = false) {
     fl.p.topk_ids = topk_ids;
     const MapSet& maps = fl.maps;
     const amoe::MoeParams& p = fl.p;
@@ -797,10 +808,8 @@ int launch_prepared(FusedLaunch& fl, void* stream, const int32_t* topk_ids = nul
         }
     }
     if (topk_ids)
-        return bmp == 32  ? launch_variant<32, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
-               : bmp == 64 ? launch_variant<64, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
-               : spc == 1  ? launch_variant<16, 1, 1, false, false, true>(maps, p, g, smem_bytes, dev, st)
-                           : launch_variant<16, 2, 1, false, false, true>(maps, p, g, smem_bytes, dev, st);
+        return write_schedule ? launch_direct<2>(maps, p, bmp, spc, g, smem_bytes, dev, st)
+                              : launch_direct<1>(maps, p, bmp, spc, g, smem_bytes, dev, st);
     if (spc == 1) {
         switch (bmp) {
             case 16: return launch_variant<16, 1>(maps, p, g, smem_bytes, dev, st);
@@ -1053,6 +1062,21 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
                                  int num_experts, int32_t* sorted_token_ids, int32_t* expert_ids,
                                  int32_t* num_tokens_post_padded, void* align_workspace, int block_m, int block_n,
                                  int warp_n, int stages, float scaling_factor, void* stream) {
+    return amoe_capi::fused_experts(hidden_states, x_fp8, x_scale, w, w_scale, w2, w2_scale, topk_ids, topk_weights, top_k, M, K, N,
+                                    num_experts, sorted_token_ids, expert_ids, num_tokens_post_padded, align_workspace, block_m,
+                                    block_n, warp_n, stages, scaling_factor, stream, true);
+}
+
+const char* alpha_moe_b200_last_error(void) { return g_last_error.c_str(); }
+const char* alpha_moe_b200_version(void) { return "alpha_moe_b200 0.1 (sm_100a)"; }
+
+}  // extern "C"
+
+int amoe_capi::fused_experts(void* hidden_states, void* x_fp8, float* x_scale, const void* w, const float* w_scale, const void* w2,
+                             const float* w2_scale, const int32_t* topk_ids, const float* topk_weights, int top_k, int M, int K,
+                             int N, int num_experts, int32_t* sorted_token_ids, int32_t* expert_ids,
+                             int32_t* num_tokens_post_padded, void* align_workspace, int block_m, int block_n, int warp_n,
+                             int stages, float scaling_factor, void* stream, bool keep_schedule) {
     if (!hidden_states || !x_fp8 || !x_scale || !topk_ids || !sorted_token_ids || !expert_ids || !num_tokens_post_padded)
         return fail(ALPHA_MOE_E_ARG, "null pointer argument");
     if (M <= 0 || top_k <= 0 || num_experts <= 0) return fail(ALPHA_MOE_E_ARG, "M, top_k and num_experts must be positive");
@@ -1074,7 +1098,7 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
     if (num_experts <= 1024 && has_direct_form(fl.plan, numel, num_experts)) {
         // Decode batches: the operator makes its schedule itself while the activations are quantised.
         if (int rc = alpha_moe_b200_per_token_group_quant_fp8(hidden_states, x_fp8, x_scale, M, K, 1, stream)) return rc;
-        return launch_prepared(fl, stream, topk_ids);
+        return launch_prepared(fl, stream, topk_ids, keep_schedule);
     }
     // extra/sglang.patch:30-31: quantise, then clear the buffer the layer accumulates into; :33-35: the schedule
     // (one launch for both when the schedule fits one CTA)
@@ -1084,9 +1108,3 @@ int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scal
         return rc;
     return launch_prepared(fl, stream);      // :38-40
 }
-
-
-const char* alpha_moe_b200_last_error(void) { return g_last_error.c_str(); }
-const char* alpha_moe_b200_version(void) { return "alpha_moe_b200 0.1 (sm_100a)"; }
-
-}  // extern "C"

@@ -10,6 +10,7 @@
 #include <torch/library.h>
 
 #include "../../include/alpha_moe_b200.h"
+#include "capi_internal.h"
 
 namespace {
 
@@ -123,13 +124,14 @@ int64_t fused_experts(const torch::Tensor& hidden, const torch::Tensor& w1, cons
     const int64_t num_post_pad = expert_ids + up((total + block_m - 1) / block_m * 4), ws = num_post_pad + 256;
     const torch::Tensor buf = at::empty({ws + ws_bytes}, hidden.options().dtype(at::kByte));
     uint8_t* const base = buf.data_ptr<uint8_t>();
-    return alpha_moe_b200_fused_experts(
+    return amoe_capi::fused_experts(        // (nobody sees this scratch: no schedule is kept in it)
         hidden.data_ptr(), base, reinterpret_cast<float*>(base + x_s), w1.data_ptr(), w1_scale.data_ptr<float>(), w2.data_ptr(),
         w2_scale.data_ptr<float>(), ids.data_ptr<int32_t>(), wts.data_ptr<float>(), static_cast<int>(top_k),
         static_cast<int>(M), static_cast<int>(K), static_cast<int>(N), static_cast<int>(E),
         reinterpret_cast<int32_t*>(base + sorted_ids), reinterpret_cast<int32_t*>(base + expert_ids),
         reinterpret_cast<int32_t*>(base + num_post_pad), ws_bytes ? base + ws : nullptr, static_cast<int>(block_m),
-        static_cast<int>(block_n), static_cast<int>(warp_n), static_cast<int>(stages), static_cast<float>(scaling_factor), stream);
+        static_cast<int>(block_n), static_cast<int>(warp_n), static_cast<int>(stages), static_cast<float>(scaling_factor), stream,
+        false);
 }
 
 }  // namespace

@@ -165,9 +165,9 @@ int alpha_moe_b200_quant_and_align(void* x_bf16, void* x_fp8, float* x_scale, in
  * hidden_states: bf16 [M,K], activations on entry, layer output on return.  Scratch, all caller-owned device
  * memory: x_fp8 [M,K] bytes, x_scale [M,K/128] f32, sorted_token_ids [M*top_k + num_experts*(block_m-1)] i32,
  * expert_ids [ceil(that / block_m)] i32, num_tokens_post_padded [1] i32, align_workspace of
- * alpha_moe_b200_align_workspace_bytes(M*top_k, num_experts) bytes (may be NULL when that is 0).  The scratch's contents are
- * unspecified on return: with block_m <= 64 and at most 8192 assignments the operator usually derives the schedule from topk_ids itself
- * and writes none of sorted_token_ids, expert_ids and num_tokens_post_padded.
+ * alpha_moe_b200_align_workspace_bytes(M*top_k, num_experts) bytes (may be NULL when that is 0).  On return (in stream order)
+ * x_fp8, x_scale, sorted_token_ids, expert_ids and num_tokens_post_padded hold what the single steps write, also where the
+ * operator makes its schedule itself (block_m <= 64 and at most 8192 assignments, usually).
  * Everything is enqueued on `stream`; nothing is allocated.  Error codes as for the single steps. */
 int alpha_moe_b200_fused_experts(void* hidden_states, void* x_fp8, float* x_scale, const void* w,
                                  const float* w_scale, const void* w2, const float* w2_scale,

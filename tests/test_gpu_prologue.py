@@ -318,6 +318,47 @@ def test_small_batches_whose_operator_makes_its_own_schedule(m, top_k, e, k, int
             assert orc.rel_l2(got.cpu(), ref) <= 2e-2
 
 
+@pytest.mark.parametrize("m,top_k,e,inter,bm,bn,stages", [
+    (1, 1, 1, 256, 16, 32, 1),             # one block and no slot behind it that an expert leaves empty
+    (1, 9, 257, 256, 16, 32, 4),           # clusters, whose blocks go from the back
+    (5, 9, 257, 256, 16, 32, 2),
+    (28, 9, 1024, 512, 8, 64, 5),          # most of the schedule lies behind the last block
+    (114, 9, 33, 256, 16, 32, 3),          # 1026 assignments; no clusters
+    (205, 10, 300, 512, 32, 64, 2),
+    (819, 10, 50, 512, 48, 64, 2),
+    (819, 10, 50, 512, 128, 64, 3),        # the schedule kernel
+])
+@pytest.mark.parametrize("routing", ["topk", "outside", "none"])
+def test_single_call_leaves_the_schedule_in_the_callers_buffers(m, top_k, e, inter, bm, bn, stages, routing):
+    """The C entry's schedule buffers hold the schedule kernel's words afterwards, whichever form the operator took."""
+    from alpha_moe_b200 import capi
+    from alpha_moe_b200.prologue import moe_align_block_size, per_token_group_quant_fp8
+    k = 256
+    g = torch.Generator().manual_seed(m + e)
+    ids = torch.stack([torch.randperm(e, generator=g)[:top_k] for _ in range(m)]).to(torch.int32)
+    if routing == "outside":
+        ids[::2, ::2] = -1
+        ids[1::2, ::3] = e
+    elif routing == "none":
+        ids[:] = e + 3
+    ids, hidden = ids.cuda(), torch.randn(m, k, generator=g).to(torch.bfloat16).cuda()
+    want = (*moe_align_block_size(ids, bm, e), *per_token_group_quant_fp8(hidden))
+    got = [torch.full_like(t.view(torch.int32), -99) for t in want[:3]] + [torch.zeros_like(t) for t in want[3:]]
+    w = torch.zeros(e, 2 * inter, k, dtype=torch.float8_e4m3fn, device="cuda")
+    w2 = torch.zeros(e, k, inter, dtype=torch.float8_e4m3fn, device="cuda")
+    ws, w2s = torch.ones(e, inter // 64, k // 128, device="cuda"), torch.ones(e, k // 128, inter // 128, device="cuda")
+    wts = torch.ones(m, top_k, device="cuda")
+    scratch = torch.empty(max(capi.align_workspace_bytes(m * top_k, e), 4), dtype=torch.uint8, device="cuda")
+    capi.fused_experts(hidden.data_ptr(), got[3].data_ptr(), got[4].data_ptr(), w.data_ptr(), ws.data_ptr(), w2.data_ptr(),
+                       w2s.data_ptr(), ids.data_ptr(), wts.data_ptr(), top_k, m, k, 2 * inter, e,
+                       got[0].data_ptr(), got[1].data_ptr(), got[2].data_ptr(), scratch.data_ptr(), bm, bn, 256 // bn, stages,
+                       1.0, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    assert capi.read_status(reset=True)[0] == 0
+    for a, b in zip(got, want):
+        assert torch.equal(a.view(torch.uint8), b.view(torch.uint8))
+
+
 def test_layer_call_refuses_cuda_tensors_in_the_words_of_the_host_checks():
     """fused_experts_impl checks CUDA tensors inside its operator: what _check_layer_arguments refuses is refused with the same
     message, an ABI error keeps its type, and the buffer is left alone."""
