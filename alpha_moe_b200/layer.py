@@ -1,9 +1,11 @@
 """The body the reference's serving patch gives `fused_experts_impl` (extra/sglang.patch:25-40), on this
 library's own kernels: knob look-up for the batch size, activation quantisation, clearing of the buffer the
 layer accumulates into, block schedule, fused operator.  `hidden_states` holds the layer output on return,
-as in the patch.  Checks, buffers and the C-ABI call are one torch operator."""
+as in the patch.  Checks, buffers and the C-ABI call are one torch operator; where only the C library has been built, the same
+three steps are taken here."""
 from __future__ import annotations
 
+import contextlib
 import os
 
 import torch
@@ -11,21 +13,10 @@ import torch
 from . import capi, load_torch_op
 from .utils import get_best_config
 
-load_torch_op()
-_fused_experts = torch.ops.alpha_moe._fused_experts.default
-
-
-@torch.compiler.disable
-def _fused_experts_outside_graphs(*args) -> int:
-    """For torch.compile: the call (in place, an error code back) stays outside its graphs."""
-    return _fused_experts(*args)
-
-
 def _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids) -> None:
     """The checks the torch operator makes on its tensors (csrc/torch_interface.cpp:58-76 of the reference, plus
-    the dtype / device / shape checks this library's operator adds), made here before any raw pointer is taken:
-    this path goes straight to the C ABI, which sees only addresses.  (CUDA tensors are checked by the same rules in
-    csrc/torch_interface.cpp.)"""
+    the dtype / device / shape checks this library's operator adds), for calls that do not get to the torch operator, which
+    checks its CUDA tensors by the same rules and in the same words (csrc/torch_interface.cpp): the C ABI sees only addresses."""
     # (written out: messages are only put together for a call that fails)
     if hidden_states.dtype != torch.bfloat16 or hidden_states.dim() != 2 or not hidden_states.is_contiguous():
         raise RuntimeError("hidden_states must be a contiguous 2-D bfloat16 tensor")
@@ -63,6 +54,51 @@ def _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weigh
     for i, t in enumerate((*weights, topk_weights, topk_ids)):
         if t.device != dev:
             raise RuntimeError(f"{('w1', 'w1_scale', 'w2', 'w2_scale', 'topk_weights', 'topk_ids')[i]} must be on {dev}")
+
+def _up(n: int) -> int:
+    return (n + 255) & ~255
+
+
+def _through_c_abi(hidden, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, block_m, block_n, warp_n, stages, scaling) -> int:
+    """What the torch operator does, on the C library alone."""
+    _check_layer_arguments(hidden, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids)
+    m, k = hidden.shape
+    e, n, _ = w1.shape
+    ids, wts = topk_ids.to(torch.int32).contiguous(), topk_weights.to(torch.float32).contiguous()
+    top_k, dev = ids.shape[1], hidden.device
+    total = m * top_k + e * (block_m - 1)
+    ws_bytes = capi.align_workspace_bytes(m * top_k, e)
+    x_s = _up(m * k)                                        # one allocation, its pieces 256-byte aligned
+    sorted_ids = x_s + _up(m * (k // 128) * 4)
+    expert_ids = sorted_ids + _up(total * 4)
+    num_post_pad = expert_ids + _up((total + block_m - 1) // block_m * 4)
+    ws = num_post_pad + 256
+    buf = torch.empty(ws + ws_bytes, dtype=torch.uint8, device=dev)
+    base = buf.data_ptr()
+    with torch.cuda.device(dev) if dev.index != torch.cuda.current_device() else contextlib.nullcontext():
+        capi.fused_experts(hidden.data_ptr(), base, base + x_s, w1.data_ptr(), w1_scale.data_ptr(), w2.data_ptr(),
+                           w2_scale.data_ptr(), ids.data_ptr(), wts.data_ptr(), top_k, m, k, n, e, base + sorted_ids,
+                           base + expert_ids, base + num_post_pad, base + ws if ws_bytes else 0, block_m, block_n, warp_n, stages,
+                           scaling, torch.cuda.current_stream(dev).cuda_stream)
+    return 0
+
+
+def _operator():
+    try:
+        load_torch_op()
+    except ImportError:
+        return _through_c_abi
+    return torch.ops.alpha_moe._fused_experts.default
+
+
+_fused_experts = _operator()
+
+
+@torch.compiler.disable
+def _fused_experts_outside_graphs(*args) -> int:
+    """For torch.compile: the call (in place, an error code back) stays outside its graphs."""
+    return _fused_experts(*args)
+
 
 def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: torch.Tensor, w2: torch.Tensor,
                        w2_scale: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,

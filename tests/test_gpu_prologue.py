@@ -410,6 +410,31 @@ def test_layer_call_refuses_cuda_tensors_in_the_words_of_the_host_checks():
     assert out is good["hidden_states"] and not out.detach().any() and out.grad_fn is None
 
 
+def test_layer_call_on_the_c_library_alone_matches_the_operator(monkeypatch):
+    """Without the torch operator's library the layer call makes its checks and buffers in Python; also on another stream, with
+    routing that has to be converted, and with the error type of the C ABI."""
+    from alpha_moe_b200 import capi, layer
+    e, k, inter, m, top_k = 8, 256, 256, 130, 8            # 1040 assignments: a workspace, too
+    g = torch.Generator().manual_seed(3)
+    dw = [t.cuda() for t in orc.make_weights(e, k, inter, g)]
+    x = torch.randn(m, k, generator=g).to(torch.bfloat16).cuda()
+    ids, wts = orc.route_topk(torch.randn(m, e, generator=g), top_k)
+    ids, wts = ids.long().cuda(), wts.double().cuda()
+    conf = dict(block_m=16, block_n=32, warp_n=8, stages=3)
+    want = layer.fused_experts_impl(x.clone(), *dw, wts, ids, config=conf)
+    monkeypatch.setattr(layer, "_fused_experts", layer._through_c_abi)
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = layer.fused_experts_impl(x.clone(), *dw, wts, ids, config=conf)
+    torch.cuda.synchronize()
+    assert orc.rel_l2(got.cpu(), want.cpu()) <= 1e-2
+    with pytest.raises(capi.AlphaMoeError, match="stages"):
+        layer.fused_experts_impl(x.clone(), *dw, wts, ids, config=dict(conf, stages=9))
+    with pytest.raises(RuntimeError, match="w1_scale"):
+        layer.fused_experts_impl(x.clone(), dw[0], dw[1][:, 1:], *dw[2:], wts, ids, config=conf)
+
+
 @pytest.mark.parametrize("backend", ["eager", "aot_eager"])
 def test_layer_call_inside_a_compiled_function(backend):
     """torch.compile breaks its graph at the layer call, as it did when the call went through ctypes."""

@@ -288,6 +288,29 @@ def test_layer_entry_checks_shapes_strides_and_dtypes_before_taking_pointers():
                            good["topk_weights"], good["topk_ids"], config=dict(block_m=16, block_n=32, warp_n=8, stages=3))
 
 
+def test_layer_module_needs_the_c_library_only(tmp_path):
+    """A tree in which the torch operator's library has not been built: alpha_moe_b200.layer imports and checks its arguments."""
+    import shutil
+    import subprocess
+    import sys
+    shutil.copytree(os.path.join(ROOT, "alpha_moe_b200"), tmp_path / "alpha_moe_b200",
+                    ignore=shutil.ignore_patterns("libalpha_moe_torch.so", "__pycache__"))
+    code = ("import torch\n"
+            "from alpha_moe_b200.layer import fused_experts_impl\n"
+            "z = torch.zeros\n"
+            "f8 = torch.float8_e4m3fn\n"
+            "a = [z(3, 256, dtype=torch.bfloat16), z(4, 256, 256, dtype=f8), z(4, 2, 2), z(4, 256, 128, dtype=f8), z(4, 2, 1),\n"
+            "     z(3, 2), z(3, 2, dtype=torch.int32)]\n"
+            "conf = dict(block_m=16, block_n=32, warp_n=8, stages=3)\n"
+            "for i, bad in ((None, 'CUDA'), (1, 'w1')):\n"
+            "    try:\n"
+            "        fused_experts_impl(*[z(4, 256, 255) if j == i else t for j, t in enumerate(a)], config=conf)\n"
+            "    except RuntimeError as err:\n"
+            "        print(bad in str(err))\n")
+    run = subprocess.run([sys.executable, "-c", code], cwd=tmp_path, capture_output=True, text=True, timeout=300)
+    assert run.stdout.split() == ["True", "True"], run.stderr
+
+
 def test_tensor_parallel_entry_points_reject_bad_arguments_before_any_launch():
     from alpha_moe_b200 import capi
     p = 0x10000
