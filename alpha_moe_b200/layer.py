@@ -112,16 +112,21 @@ def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: 
     if not hidden_states.is_cuda:
         _check_layer_arguments(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids)
         raise RuntimeError("hidden_states must be a CUDA tensor (there is no CPU implementation)")
-    if isinstance(config, dict):
-        conf = config
-    else:
-        path = config or os.getenv("ALPHA_MOE_CONFIG")
-        if not path:
-            raise RuntimeError("no knob table: pass config= or set ALPHA_MOE_CONFIG")
-        conf = get_best_config(path, hidden_states.size(0))
+    args = (hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids)
+    try:
+        if isinstance(config, dict):
+            conf = config
+        else:
+            path = config or os.getenv("ALPHA_MOE_CONFIG")
+            if not path:
+                raise RuntimeError("no knob table: pass config= or set ALPHA_MOE_CONFIG")
+            conf = get_best_config(path, hidden_states.size(0))
+        knobs = conf["block_m"], conf["block_n"], conf["warp_n"], conf["stages"]
+    except Exception:
+        _check_layer_arguments(*args)        # a tensor that is refused comes before a table that is not there
+        raise
     call = _fused_experts_outside_graphs if torch.compiler.is_compiling() else _fused_experts
-    rc = call(hidden_states, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, conf["block_m"], conf["block_n"],
-              conf["warp_n"], conf["stages"], float(routed_scaling_factor or 1.0))
+    rc = call(*args, *knobs, float(routed_scaling_factor or 1.0))
     if rc != 0:
         capi._check(rc)
     return hidden_states

@@ -288,6 +288,32 @@ def test_layer_entry_checks_shapes_strides_and_dtypes_before_taking_pointers():
                            good["topk_weights"], good["topk_ids"], config=dict(block_m=16, block_n=32, warp_n=8, stages=3))
 
 
+def test_a_refused_tensor_comes_before_a_refused_knob_table(tmp_path):
+    """CUDA tensors are checked behind the knob look-up, inside the operator; a look-up that fails must not hide what the checks say.
+    (Fake CUDA tensors: nothing is launched.)"""
+    from torch._subclasses.fake_tensor import FakeTensorMode
+    from alpha_moe_b200.layer import fused_experts_impl
+    table = os.path.join(ROOT, "configs", "moe_b200_E257_I256_K7168.json")
+    conf = dict(block_m=16, block_n=32, warp_n=8, stages=3)
+    f8 = torch.float8_e4m3fn
+    with FakeTensorMode():
+        def z(*shape, dtype=torch.float32):
+            return torch.empty(shape, dtype=dtype, device="cuda")
+
+        def make(w1_k=256, shape=(3, 256)):
+            return (z(*shape, dtype=torch.bfloat16), z(4, 256, w1_k, dtype=f8), z(4, 2, 2), z(4, 256, 128, dtype=f8), z(4, 2, 1), z(3, 2), z(3, 2, dtype=torch.int32))
+
+        with pytest.raises(RuntimeError, match="2-D"):
+            fused_experts_impl(*make(shape=()), config=table)
+        for config in (str(tmp_path / "no_such_table.json"), {k: v for k, v in conf.items() if k != "stages"}):
+            with pytest.raises(RuntimeError, match="w1"):
+                fused_experts_impl(*make(w1_k=128), config=config)
+        with pytest.raises(FileNotFoundError):
+            fused_experts_impl(*make(), config=str(tmp_path / "no_such_table.json"))
+        with pytest.raises(KeyError):
+            fused_experts_impl(*make(), config={})
+
+
 def test_layer_module_needs_the_c_library_only(tmp_path):
     """A tree in which the torch operator's library has not been built: alpha_moe_b200.layer imports and checks its arguments."""
     import shutil
