@@ -73,6 +73,12 @@ def _check(rc: int) -> None:
         raise AlphaMoeError(f"alpha_moe_b200 error {rc}: {last_error()}")
 
 
+def error_of(err: RuntimeError) -> RuntimeError:
+    """An error of this library that a torch operator raised, with the type of the C ABI's errors; any other as it is."""
+    text = str(err)
+    return AlphaMoeError(text.splitlines()[0]) if text.startswith("alpha_moe_b200 error ") else err
+
+
 def fused_moe_w8a8_up_down(x, x_scale, w, w_scale, w2, w2_scale, out, sorted_token_ids, expert_ids,
                            num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, sorted_num,
                            block_m, block_n, warp_n, stages, scaling_factor, stream=0) -> None:

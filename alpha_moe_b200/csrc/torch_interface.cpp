@@ -80,13 +80,13 @@ void fused_moe_w8a8_up_down(const torch::Tensor& x, const torch::Tensor& x_scale
 
 // The layer call (alpha_moe_b200/layer.py: fused_experts_impl) behind its knob look-up: the same tensor checks in the same order and
 // words as _check_layer_arguments there, one allocation for all intermediate buffers (256-byte aligned pieces), one call of
-// the C ABI, whose error code it returns.  An eager call of one token is bound by its host time, and two dozen tensor
-// attributes read from Python, nine addresses and a foreign-function call with 24 arguments were most of it (DeepSeek-V3 TP8
-// shard, one token, calls in a row, 23.2 -> 20.5 us; the same call from a graph takes 18.5).
-int64_t fused_experts(const torch::Tensor& hidden, const torch::Tensor& w1, const torch::Tensor& w1_scale,
-                      const torch::Tensor& w2, const torch::Tensor& w2_scale, const torch::Tensor& topk_weights,
-                      const torch::Tensor& topk_ids, int64_t block_m, int64_t block_n, int64_t warp_n, int64_t stages,
-                      double scaling_factor) {
+// the C library, whose error it raises in the words that alpha_moe_b200/capi.py knows again.  (It returns nothing: the tracer of
+// torch.jit.trace, which records the call, takes no number as a result.)  An eager call of one token is bound by its host time,
+// and two dozen tensor attributes read from Python, nine addresses and a foreign-function call with 24 arguments were most of it
+// (DeepSeek-V3 TP8 shard, one token, calls in a row, 23.2 -> 20.5 us; the same call from a graph takes 18.5).
+void fused_experts(const torch::Tensor& hidden, const torch::Tensor& w1, const torch::Tensor& w1_scale, const torch::Tensor& w2,
+                   const torch::Tensor& w2_scale, const torch::Tensor& topk_weights, const torch::Tensor& topk_ids,
+                   int64_t block_m, int64_t block_n, int64_t warp_n, int64_t stages, double scaling_factor) {
     const at::AutoDispatchBelowADInplaceOrView below;      // nothing here is recorded, whoever requires gradients
     TORCH_CHECK(hidden.scalar_type() == at::kBFloat16 && hidden.dim() == 2 && hidden.is_contiguous(),
                 "hidden_states must be a contiguous 2-D bfloat16 tensor");
@@ -124,7 +124,7 @@ int64_t fused_experts(const torch::Tensor& hidden, const torch::Tensor& w1, cons
     const int64_t num_post_pad = expert_ids + up((total + block_m - 1) / block_m * 4), ws = num_post_pad + 256;
     const torch::Tensor buf = at::empty({ws + ws_bytes}, hidden.options().dtype(at::kByte));
     uint8_t* const base = buf.data_ptr<uint8_t>();
-    return amoe_capi::fused_experts(        // (nobody sees this scratch: no schedule is kept in it)
+    const int rc = amoe_capi::fused_experts(        // (nobody sees this scratch: no schedule is kept in it)
         hidden.data_ptr(), base, reinterpret_cast<float*>(base + x_s), w1.data_ptr(), w1_scale.data_ptr<float>(), w2.data_ptr(),
         w2_scale.data_ptr<float>(), ids.data_ptr<int32_t>(), wts.data_ptr<float>(), static_cast<int>(top_k),
         static_cast<int>(M), static_cast<int>(K), static_cast<int>(N), static_cast<int>(E),
@@ -132,6 +132,7 @@ int64_t fused_experts(const torch::Tensor& hidden, const torch::Tensor& w1, cons
         reinterpret_cast<int32_t*>(base + num_post_pad), ws_bytes ? base + ws : nullptr, static_cast<int>(block_m),
         static_cast<int>(block_n), static_cast<int>(warp_n), static_cast<int>(stages), static_cast<float>(scaling_factor), stream,
         false);
+    TORCH_CHECK(rc == ALPHA_MOE_OK, "alpha_moe_b200 error ", rc, ": ", alpha_moe_b200_last_error());
 }
 
 }  // namespace
@@ -159,7 +160,7 @@ TORCH_LIBRARY_FRAGMENT(alpha_moe, m) {
         ") -> ()");
     m.impl("fused_moe_w8a8_up_down", torch::kCUDA, &fused_moe_w8a8_up_down);
     m.def("_fused_experts(Tensor(a!) hidden, Tensor w1, Tensor w1_scale, Tensor w2, Tensor w2_scale, Tensor topk_weights, "
-          "Tensor topk_ids, int block_m, int block_n, int warp_n, int stages, float scaling_factor) -> int");
+          "Tensor topk_ids, int block_m, int block_n, int warp_n, int stages, float scaling_factor) -> ()");
     m.impl("_fused_experts", torch::kCUDA, &fused_experts);
     m.impl("_fused_experts", torch::dispatch(c10::DispatchKey::AutogradCUDA, TORCH_FN(fused_experts)));
 }

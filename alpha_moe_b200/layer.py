@@ -59,7 +59,7 @@ def _up(n: int) -> int:
     return (n + 255) & ~255
 
 
-def _through_c_abi(hidden, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, block_m, block_n, warp_n, stages, scaling) -> int:
+def _through_c_abi(hidden, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, block_m, block_n, warp_n, stages, scaling) -> None:
     """What the torch operator does, on the C library alone."""
     _check_layer_arguments(hidden, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids)
     m, k = hidden.shape
@@ -80,7 +80,6 @@ def _through_c_abi(hidden, w1, w1_scale, w2, w2_scale, topk_weights, topk_ids, b
                            w2_scale.data_ptr(), ids.data_ptr(), wts.data_ptr(), top_k, m, k, n, e, base + sorted_ids,
                            base + expert_ids, base + num_post_pad, base + ws if ws_bytes else 0, block_m, block_n, warp_n, stages,
                            scaling, torch.cuda.current_stream(dev).cuda_stream)
-    return 0
 
 
 def _operator():
@@ -95,9 +94,9 @@ _fused_experts = _operator()
 
 
 @torch.compiler.disable
-def _fused_experts_outside_graphs(*args) -> int:
-    """For torch.compile: the call (in place, an error code back) stays outside its graphs."""
-    return _fused_experts(*args)
+def _fused_experts_outside_graphs(*args) -> None:
+    """For torch.compile: the call (in place) stays outside its graphs."""
+    _fused_experts(*args)
 
 
 def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: torch.Tensor, w2: torch.Tensor,
@@ -126,7 +125,8 @@ def fused_experts_impl(hidden_states: torch.Tensor, w1: torch.Tensor, w1_scale: 
         _check_layer_arguments(*args)        # a tensor that is refused comes before a table that is not there
         raise
     call = _fused_experts_outside_graphs if torch.compiler.is_compiling() else _fused_experts
-    rc = call(*args, *knobs, float(routed_scaling_factor or 1.0))
-    if rc != 0:
-        capi._check(rc)
+    try:
+        call(*args, *knobs, float(routed_scaling_factor or 1.0))
+    except RuntimeError as err:
+        raise capi.error_of(err)
     return hidden_states

@@ -455,3 +455,24 @@ def test_layer_call_inside_a_compiled_function(backend):
     h = x.clone()
     got = torch.compile(layer, backend=backend)(h)
     assert orc.rel_l2(got.cpu(), want.cpu()) <= 1e-2 and orc.rel_l2(2 * h.cpu(), want.cpu()) <= 1e-2
+
+
+def test_layer_call_inside_a_traced_function():
+    """torch.jit.trace records the layer call: the trace computes the layer on other activations and another routing."""
+    from alpha_moe_b200.layer import fused_experts_impl
+    e, k, inter, m, top_k = 8, 256, 256, 5, 2
+    g = torch.Generator().manual_seed(11)
+    dw = [t.cuda() for t in orc.make_weights(e, k, inter, g)]
+    conf = dict(block_m=16, block_n=32, warp_n=8, stages=3)
+
+    def layer(h, wts, ids):
+        return fused_experts_impl(h, *dw, wts, ids, routed_scaling_factor=2.5, config=conf) * 2
+
+    def inputs():
+        ids, wts = orc.route_topk(torch.randn(m, e, generator=g), top_k)
+        return torch.randn(m, k, generator=g).to(torch.bfloat16).cuda(), wts.cuda(), ids.cuda()
+
+    traced = torch.jit.trace(layer, inputs(), check_trace=False)
+    h, wts, ids = inputs()
+    want = layer(h.clone(), wts, ids)
+    assert orc.rel_l2(traced(h, wts, ids).cpu(), want.cpu()) <= 1e-2

@@ -314,6 +314,18 @@ def test_a_refused_tensor_comes_before_a_refused_knob_table(tmp_path):
             fused_experts_impl(*make(), config={})
 
 
+def test_the_layer_calls_operator_can_be_recorded():
+    """torch.jit.trace passes every operator that it records through a function that takes tensors and nothing as results; an operator
+    that returns a number stops it.  The errors of the C library keep their type across the operator."""
+    import alpha_moe_b200
+    from alpha_moe_b200 import capi
+    alpha_moe_b200.load_torch_op()
+    assert str(torch.ops.alpha_moe._fused_experts.default._schema).endswith("-> ()")
+    mine, other = RuntimeError("alpha_moe_b200 error -1: stages must be\nC++ trace"), RuntimeError("w1 must be contiguous")
+    assert isinstance(capi.error_of(mine), capi.AlphaMoeError) and str(capi.error_of(mine)) == "alpha_moe_b200 error -1: stages must be"
+    assert capi.error_of(other) is other
+
+
 def test_layer_module_needs_the_c_library_only(tmp_path):
     """A tree in which the torch operator's library has not been built: alpha_moe_b200.layer imports and checks its arguments."""
     import shutil
