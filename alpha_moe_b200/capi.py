@@ -56,6 +56,8 @@ lib.alpha_moe_b200_selftest_wait_timeout.restype = _i
 lib.alpha_moe_b200_selftest_wait_timeout.argtypes = [_i, _i, _i, _vp, _vp]
 lib.alpha_moe_b200_selftest_warp_wait.restype = _i
 lib.alpha_moe_b200_selftest_warp_wait.argtypes = [_i, _vp, _vp]
+lib.alpha_moe_b200_selftest_closing_wait.restype = _i
+lib.alpha_moe_b200_selftest_closing_wait.argtypes = [_i, _vp, _vp]
 lib.alpha_moe_b200_last_error.restype = ctypes.c_char_p
 lib.alpha_moe_b200_version.restype = ctypes.c_char_p
 
@@ -180,6 +182,11 @@ def selftest_wait_timeout(limit_cycles: int, where: int, iter_: int, result2, st
 def selftest_warp_wait(limit_cycles: int, result5, stream=0) -> None:
     """Launches the self-test of the whole-warp waits; result5 = device address of five int32 (ballots of the answers)."""
     _check(lib.alpha_moe_b200_selftest_warp_wait(limit_cycles, result5, stream))
+
+
+def selftest_closing_wait(limit_cycles: int, result3, stream=0) -> None:
+    """Launches the self-test of a CTA's last wait; result3 = device address of three int32 (what the waits returned)."""
+    _check(lib.alpha_moe_b200_selftest_closing_wait(limit_cycles, result3, stream))
 
 
 def read_status(reset: bool = False):

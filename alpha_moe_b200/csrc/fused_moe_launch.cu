@@ -383,6 +383,32 @@ __global__ void warp_wait_selftest_kernel(amoe::KernelStatus* status, unsigned* 
     }
 }
 
+// Self-test of the wait that a CTA which gives up makes last.  The abort flag is raised all along.  result[0] = what an ordinary wait
+// answers (0, at its first look at the flag), [1] = the last wait while an arrival on the second of its barriers is still to come
+// (1), [2] = the same with barriers that nothing arrives on (0, after the limit).
+__global__ void closing_wait_selftest_kernel(amoe::KernelStatus* status, int* result, long long limit_cycles) {
+    __shared__ uint64_t bars[2];
+    __shared__ int abort_flag;
+    if (threadIdx.x == 0) {
+        amoe::mbar_init(&bars[0], 1);
+        amoe::mbar_init(&bars[1], 1);
+        abort_flag = 1;
+        amoe::fence_mbar_init();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        result[0] = amoe::mbar_wait(&bars[1], 0, &abort_flag, status, 0, 0);
+        result[2] = amoe::mbar_wait_either_limit(&bars[0], &bars[0], limit_cycles);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) result[1] = amoe::mbar_wait_either_limit(&bars[0], &bars[1], 100 * limit_cycles);
+    if (threadIdx.x == 32) {
+        const long long t0 = clock64();
+        while (clock64() - t0 < limit_cycles) {}
+        amoe::mbar_arrive(&bars[1]);
+    }
+}
+
 std::atomic<int> g_ksplit_override{0};     // 0 = automatic; set through alpha_moe_b200_set_ksplit (tuners, tests)
 
 // Clusters of CTAs along K for small batches (narrow tile, one slice per CTA only): the largest cluster size for
@@ -994,6 +1020,19 @@ int alpha_moe_b200_selftest_warp_wait(int limit_cycles, int32_t* result5, void* 
     if (int rc = device_facts(dev, &facts)) return rc;
     warp_wait_selftest_kernel<<<1, 32, 0, static_cast<cudaStream_t>(stream)>>>(facts.status, reinterpret_cast<unsigned*>(result5),
                                                                             limit_cycles);
+    CUDA_TRY(cudaGetLastError());
+    return ALPHA_MOE_OK;
+}
+
+int alpha_moe_b200_selftest_closing_wait(int limit_cycles, int32_t* result3, void* stream) {
+    if (!result3) return fail(ALPHA_MOE_E_ARG, "result3 is null");
+    if (limit_cycles < 1000 || limit_cycles > 2000000)
+        return fail(ALPHA_MOE_E_ARG, "limit_cycles must be in 1000..2000000 (about 1 ms), got %d", limit_cycles);
+    int dev = 0;
+    CUDA_TRY(cudaGetDevice(&dev));
+    DeviceFacts facts;
+    if (int rc = device_facts(dev, &facts)) return rc;
+    closing_wait_selftest_kernel<<<1, 64, 0, static_cast<cudaStream_t>(stream)>>>(facts.status, result3, limit_cycles);
     CUDA_TRY(cudaGetLastError());
     return ALPHA_MOE_OK;
 }

@@ -124,6 +124,15 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, v
                                                KernelStatus* status, int where, int iter) {
     return mbar_wait_warp_limit(bar, parity, abort_flag, status, where, iter, kWaitLimitCycles);
 }
+// The last wait of a CTA that gives up: first phase of either of two mbarriers, or `limit_cycles`, whatever the abort flag says.
+__device__ __forceinline__ bool mbar_wait_either_limit(uint64_t* a, uint64_t* b, long long limit_cycles) {
+    const long long t0 = clock64();
+    for (;;) {
+        if (mbar_try_wait(a, 0) || mbar_try_wait(b, 0)) return true;
+        if (clock64() - t0 > limit_cycles) return false;
+    }
+}
+constexpr long long kLandingCycles = 2000000LL;      // about a millisecond: a thousand times what a store to a peer takes
 // A whole warp waits until the counter `turn` in shared memory has reached `it`; one answer for all lanes, as above.
 __device__ __forceinline__ bool turn_wait_warp_limit(volatile int* turn, int it, volatile int* abort_flag,
                                                      KernelStatus* status, int where, long long limit_cycles) {
@@ -154,8 +163,9 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The same without any ordering of memory accesses: at the end of a kernel, where no CTA may go while a peer still writes
-// into or reads from its shared memory.  (A releasing arrival would wait for the acknowledgement of all reductions.)
+// The same without any ordering of memory accesses: at the end of a kernel, where no CTA may go while a peer may still issue writes
+// into or reads from its shared memory.  (A releasing arrival would wait for the acknowledgement of all reductions.)  Writes that a
+// peer has issued are not waited for: their receiver does that on the mbarrier that counts them.
 __device__ __forceinline__ void cluster_sync_all_relaxed() {
     asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }

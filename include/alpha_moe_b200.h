@@ -196,6 +196,11 @@ int alpha_moe_b200_selftest_wait_timeout(int limit_cycles, int where, int iter, 
  * (1000..200000000), so the status word is set as above (where = 50); the kernel returns normally. */
 int alpha_moe_b200_selftest_warp_wait(int limit_cycles, int32_t* result5, void* stream);
 
+/* Self-test of the wait with which a CTA that gave up stays for what its cluster's peers have sent it: the abort flag does not end
+ * it, an arrival does, and so does its limit.  result3 (device, 3 x int32) receives {0, 1, 0}: an ordinary wait under a raised abort
+ * flag, the last wait while an arrival is still to come, the same without one.  limit_cycles in 1000..2000000. */
+int alpha_moe_b200_selftest_closing_wait(int limit_cycles, int32_t* result3, void* stream);
+
 /* What the launcher uses for a problem and a knob tuple; for tuners and tests.  It runs the launcher's own
  * planning code.  num_blocks = schedule blocks as the launcher counts them: for block_m <= 64 those that can be live at most,
  * min(ceil(sorted_num / block_m), M * top_k), which decide ksplit; for block_m > 64 those that are live at least,

@@ -52,6 +52,25 @@ def test_lanes_that_see_different_things_still_get_one_answer():
     assert capi.read_status(reset=True) == (1, 0, 50, 0)          # the first wait to run out is the one on record
 
 
+def test_a_cta_that_gave_up_stays_for_what_its_peers_have_sent():
+    """On the way out of a cluster after a wait ran out, stores and arrivals of the peers may still be under way to the CTA's shared
+    memory.  Its last wait goes on under a raised abort flag until they have landed, and no longer than its limit."""
+    from alpha_moe_b200 import capi
+    assert capi.read_status(reset=True)[0] == 0
+    res = torch.full((3,), 7, dtype=torch.int32, device="cuda")
+    t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    t0.record()
+    capi.selftest_closing_wait(200_000, res.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    t1.record()
+    torch.cuda.synchronize()
+    assert res.tolist() == [0, 1, 0]
+    assert t0.elapsed_time(t1) < 50.0
+    assert capi.read_status(reset=True)[0] == 0           # nothing of this is an event of its own
+    for bad in (0, 2_000_001):
+        with pytest.raises(capi.AlphaMoeError):
+            capi.selftest_closing_wait(bad, res.data_ptr())
+
+
 @pytest.mark.parametrize("which", ["barrier", "exchange_sum", "allreduce", "reduce_scatter"])
 def test_cross_gpu_wait_runs_out_when_a_rank_never_arrives(which):
     """The tensor-parallel exchange kernels wait for the other ranks through flag words in peer-mapped memory.  Here
