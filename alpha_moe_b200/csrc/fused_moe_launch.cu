@@ -740,19 +740,12 @@ int plan_fused(const DeviceFacts& facts, int M, int top_k, int K, int N, int sor
 // (227 KB per SM less 1 KB reserved per CTA leaves 113 KB of dynamic shared memory for each).
 bool pair64(const FusedPlan& fp) { return fp.bmp == 64 && fp.depth <= 2 && fp.smem_bytes <= kPairDynSmem; }
 
-// Whether the launch has a DIRECT form: the tiles of 16 tokens, and the wider ones with two slices where they have the fragment
-// epilogue's usual form and one epilogue warpgroup.
-bool has_direct_form(const FusedPlan& fp, long long numel, int num_experts) {
-    const bool shape = fp.bmp == 16 || (fp.spc == 2 && fp.depth >= 2 && (fp.bmp == 32 || pair64(fp)));
-    return shape && numel <= amoe::kDirectMax && amoe::direct_bytes(num_experts) <= fp.spc * fp.bmp * 128;
-}
-
 // One launch of the operator, checked and planned: nothing but a CUDA error can refuse it any more.
 struct FusedLaunch {
     MapSet maps;
     amoe::MoeParams p;
     FusedPlan plan;
-    int grid, dev;
+    int grid, dev, sms;
 };
 int prepare_fused(const void* x, const float* x_scale, const void* w, const float* w_scale, const void* w2,
                   const float* w2_scale, void* const* outs, int tp_world, int tp_rank, const int32_t* sorted_token_ids,
@@ -803,7 +796,32 @@ int prepare_fused(const void* x, const float* x_scale, const void* w, const floa
     const long long grid = fp.nblocks * (N / 256 / fp.spc) * fp.ksplit;
     if (grid > 0x7FFFFFFFLL) return fail(ALPHA_MOE_E_ARG, "grid too large");
     fl->grid = static_cast<int>(grid);
+    fl->sms = facts.sms;
     return ALPHA_MOE_OK;
+}
+
+// Whether a layer call takes the operator's DIRECT form: tiles of 16 tokens, and the wider ones with two slices where they have the
+// fragment epilogue's usual form and one epilogue warpgroup.  The form saves the schedule kernel, what the call waits for beside
+// it and the latency of reading its result, once per call.  It costs every CTA two readings of all ids, 256 at a time, and every
+// CTA without a block (the grid is what the routing might need) the same before it can leave; only the first round of CTAs hides
+// that behind the quantiser.  So the line is at eight rounds of two CTAs per SM.  Eager layer calls in a row, schedule kernel -> direct
+// form, uniform / Zipf(1.2) routing, by the grid's rounds:
+//   DeepSeek-V3 TP8 shard: 203 tokens (1.2) 232.0 -> 226.9 / 189.9 -> 184.9 us, 300 (1.4) 241.6 -> 228.3 / 287.3 -> 274.7, 500 (1.3)
+//   241.3 -> 233.5 / 307.9 -> 299.9, 700 (1.5) 254.5 -> 246.2 / 316.4 -> 305.8, in blocks of 48 777 (1.3) 271.4 -> 265.6 / 367.3 ->
+//   370.8 and 910 (1.4) 280.2 -> 273.1 / 365.6 -> 367.6;
+//   Qwen3-Next shard: 96 tokens (1.9) 116.9 -> 112.8 / 66.3 -> 62.3, 300 (2.8) 146.9 -> 132.9 / 143.3 -> 134.7, 600 (2.9) 147.3 -> 138.5 /
+//   152.8 -> 150.5, 819 (2.5) 152.1 -> 144.6 / 161.6 -> 160.5;
+//   unsharded DeepSeek-V3 layer: 9 tokens (4.4) 430.4 -> 426.5 / 295.9 -> 294.4, 16 (7.8) 654.5 -> 651.5 / 417.7 -> 415.6, 24 (5.8) 877 ->
+//   878 / 524 -> 525, 64 (8.03) 1431 -> 1430 / 883 -> 891, 100 (8.1) 1575 -> 1566 / 1015 -> 1027, 203 (9.6) 1751 -> 1747 / 1498 -> 1499,
+//   400 (9.8) 1820 -> 1819 / 1725 -> 1735, 640 (12) 1890 -> 1892 / 2025 -> 2048, 910 (11) 2007 -> 2028 / 2284 -> 2326.
+// From a graph, where the schedule beside the quantiser costs less than in an eager call, the form still gains at 500 tokens
+// (Qwen3-Next 136.4 -> 131.6 / 140.6 -> 140.2) and loses some at the end of its range (819 tokens 140.1 -> 139.6 / 155.8 -> 159.0);
+// batches of that size are not what graphs are captured for.
+bool has_direct_form(const FusedLaunch& fl, long long numel, int num_experts) {
+    const FusedPlan& fp = fl.plan;
+    const bool shape = fp.bmp == 16 || (fp.spc == 2 && fp.depth >= 2 && (fp.bmp == 32 || pair64(fp)));
+    return shape && numel <= amoe::kDirectMax && fl.grid <= 8 * 2 * fl.sms &&
+           amoe::direct_bytes(num_experts) <= fp.spc * fp.bmp * 128;
 }
 
 // topk_ids: the batch's routing for a launch that takes it instead of a schedule (has_direct_form), else null; write_schedule: such
@@ -1134,7 +1152,7 @@ int amoe_capi::fused_experts(void* hidden_states, void* x_fp8, float* x_scale, c
                                num_tokens_post_padded, topk_weights, top_k, M, K, N, num_experts, static_cast<int>(sorted_num),
                                block_m, block_n, warp_n, stages, scaling_factor, &fl))
         return rc;
-    if (num_experts <= 1024 && has_direct_form(fl.plan, numel, num_experts)) {
+    if (num_experts <= 1024 && has_direct_form(fl, numel, num_experts)) {
         // Decode batches: the operator makes its schedule itself while the activations are quantised.
         if (int rc = alpha_moe_b200_per_token_group_quant_fp8(hidden_states, x_fp8, x_scale, M, K, 1, stream)) return rc;
         return launch_prepared(fl, stream, topk_ids, keep_schedule);

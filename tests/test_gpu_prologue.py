@@ -476,3 +476,47 @@ def test_layer_call_inside_a_traced_function():
     h, wts, ids = inputs()
     want = layer(h.clone(), wts, ids)
     assert orc.rel_l2(traced(h, wts, ids).cpu(), want.cpu()) <= 1e-2
+
+
+@pytest.mark.parametrize("m,top_k,e,inter,bm,bn,stages,own", [
+    (1, 1, 1, 256, 16, 32, 1, True),
+    (97, 9, 257, 2048, 16, 64, 2, True),         # eight slice groups: 2368 CTAs, the line on 148 SMs
+    (98, 9, 257, 2048, 16, 64, 2, False),
+    (1024, 8, 2, 256, 32, 64, 2, True),          # 8192 assignments
+    (1025, 8, 2, 256, 32, 64, 2, False),
+    (33, 9, 40, 256, 32, 32, 2, False),          # a tile of 32 with one slice, one with a ring of one slot
+    (33, 9, 40, 256, 32, 64, 1, False),
+    (33, 9, 40, 256, 40, 64, 2, True),           # a tile of 64 with the short ring, with a longer one
+    (33, 9, 40, 256, 40, 64, 3, False),
+    (33, 9, 871, 128, 16, 32, 3, False),         # more experts than the histogram has room for
+])
+def test_which_layer_calls_make_their_own_schedule(m, top_k, e, inter, bm, bn, stages, own):
+    """Both sides of every line between the operator that makes its own schedule and the schedule kernel, each against the steps
+    one by one, token by token."""
+    from torch.profiler import ProfilerActivity, profile
+    from alpha_moe_b200 import capi
+    from alpha_moe_b200.layer import fused_experts_impl
+    from alpha_moe_b200.prologue import moe_align_block_size, per_token_group_quant_fp8
+    k = 128
+    g = torch.Generator(device="cuda").manual_seed(m + e)
+    w = torch.randn(e, 2 * inter, k, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    w2 = torch.randn(e, k, inter, generator=g, device="cuda").to(torch.float8_e4m3fn)
+    ws = torch.rand(e, inter // 64, 1, generator=g, device="cuda") * 0.02 + 0.01
+    w2s = torch.rand(e, 1, inter // 128, generator=g, device="cuda") * 0.02 + 0.01
+    ids = torch.randint(0, e, (m, top_k), generator=g, device="cuda", dtype=torch.int32)
+    wts = torch.rand(m, top_k, generator=g, device="cuda") + 0.1
+    hidden = torch.randn(m, k, generator=g, device="cuda").to(torch.bfloat16)
+    conf = {"block_m": bm, "block_n": bn, "warp_n": 256 // bn, "stages": stages}
+    xq, xs = per_token_group_quant_fp8(hidden)
+    sid, eid, npp = moe_align_block_size(ids, bm, e)
+    want = torch.zeros_like(hidden)
+    torch.ops.alpha_moe.fused_moe_w8a8_up_down(xq, xs, w, ws, w2, w2s, sid, eid, npp, wts, want, top_k, bm, bn, 256 // bn, stages, 1.0)
+    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+        fused_experts_impl(hidden, w, ws, w2, w2s, wts, ids, config=conf)
+        torch.cuda.synchronize()
+    names = [ev.key for ev in prof.key_averages()]
+    assert any("fused_moe" in n for n in names), names
+    assert any("align" in n for n in names) != own, names
+    assert capi.read_status(reset=True)[0] == 0
+    err = (hidden.float() - want.float()).norm(dim=1) / want.float().norm(dim=1)
+    assert float(err.max()) <= 2e-2
