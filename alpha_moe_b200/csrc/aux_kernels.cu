@@ -599,6 +599,8 @@ int alpha_moe_b200_per_token_group_quant_fp8(void* x_bf16, void* x_fp8, float* x
     AUX_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     long long blocks = (n_groups + 31) / 32;
     if (blocks > static_cast<long long>(sms) * 8) blocks = static_cast<long long>(sms) * 8;
+    // In ordinary stream order, and that has to stay: the operator behind it may start as soon as this kernel has, and the forms that
+    // make their own schedule then read the routing, which whatever is in front of this kernel may have written.
     group_quant_fp8_kernel<<<static_cast<unsigned>(blocks), 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<__nv_bfloat16*>(x_bf16), static_cast<uint8_t*>(x_fp8), x_scale, n_groups, zero_src);
     AUX_TRY(cudaGetLastError());

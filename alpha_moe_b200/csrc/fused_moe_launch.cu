@@ -190,9 +190,11 @@ int ensure_smem_attr(Kern kern, std::atomic<int>* configured, int dev) {
     return ALPHA_MOE_OK;
 }
 
-// Every fused kernel is launched with programmatic stream serialisation: its CTAs may be scheduled while the kernel
-// in front of it in the stream is finishing (this library's quantise / schedule kernels say when), and its first
-// statement is the wait for that kernel's completion - so launch latency overlaps the predecessor instead of following it.
+// Every fused kernel is launched with programmatic stream serialisation: its CTAs may be scheduled while the kernel in front of it in
+// the stream is finishing (this library's quantise / schedule kernels say when), so launch latency overlaps the predecessor instead of
+// following it.  The forms that take a schedule wait for that kernel's completion in their first statement.  The DIRECT forms read
+// routing, weights and block scales before they wait: that needs a kernel in front which started only when everything before it was
+// complete, i.e. one launched in ordinary stream order (the quantiser, in aux_kernels.cu).
 template <typename Kern>
 int launch_dependent(Kern kern, int grid, int threads, int smem_bytes, int cluster, cudaStream_t stream, const MapSet& maps,
                      const amoe::MoeParams& p) {

@@ -683,6 +683,8 @@ def main():
                                wl.w2.data_ptr(), wl.w2_scale.data_ptr(), ids.data_ptr(), wts.data_ptr(), sh.top_k, m, sh.k,
                                2 * sh.inter, sh.e, sid.data_ptr(), eid.data_ptr(), npp.data_ptr(), ws.data_ptr(), bm, bn, wn,
                                st, sh.scaling, stream)
+        # up to 8192 assignments the operator makes its schedule itself, above it the schedule kernel runs beside the quantiser
+        per_call = 2 if numel <= 8192 else 3
         tot = 0.0
         for i in range(warmup + steps):
             hs.copy_(x0)
@@ -694,10 +696,10 @@ def main():
             torch.cuda.synchronize()
             if i >= warmup:
                 tot += e0.elapsed_time(e1)
-        launches[0] += 3 * steps
+        launches[0] += per_call * steps
         if m > GRAPH_MAX_M:
             return tot / steps, None
-        # the same sequence replayed from a CUDA graph (the three launches of the eager call are host-bound at this size)
+        # the same sequence replayed from a CUDA graph (the launches of the eager call are host-bound at this size)
         s_ = torch.cuda.Stream()
         s_.wait_stream(torch.cuda.current_stream())
         g = torch.cuda.CUDAGraph()
@@ -716,7 +718,7 @@ def main():
             e1.record()
             torch.cuda.synchronize()
             gtot += e0.elapsed_time(e1)
-        launches[0] += 3 * steps
+        launches[0] += per_call * steps
         return tot / steps, gtot / steps
 
     def time_e2e(wl, m, steps, warmup):
