@@ -1,6 +1,8 @@
 """GPU tests of the two pre-operator kernels, bit-exact against the CPU restatement (integer and
 byte work): block schedule and per-token-group fp8 quantisation, then the whole call-site sequence
 of extra/sglang.patch:25-41 end to end."""
+import re
+
 import pytest
 import torch
 
@@ -605,12 +607,17 @@ def test_which_layer_calls_make_their_own_schedule(m, top_k, e, inter, bm, bn, s
     sid, eid, npp = moe_align_block_size(ids, bm, e)
     want = torch.zeros_like(hidden)
     torch.ops.alpha_moe.fused_moe_w8a8_up_down(xq, xs, w, ws, w2, w2s, sid, eid, npp, wts, want, top_k, bm, bn, 256 // bn, stages, 1.0)
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        fused_experts_impl(hidden, w, ws, w2, w2s, wts, ids, config=conf)
-        torch.cuda.synchronize()
-    names = [ev.key for ev in prof.key_averages()]
-    assert any("fused_moe" in n for n in names), names
-    assert any("align" in n for n in names) != own, names
+    form = None
+    for _ in range(4):                       # (the profiler loses a kernel's record now and then)
+        got = hidden.clone()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            fused_experts_impl(got, w, ws, w2, w2s, wts, ids, config=conf)
+            torch.cuda.synchronize()
+        names = [ev.key for ev in prof.key_averages()]
+        form = next((mt.group(1) for mt in (re.search(r"sm100_kernel<.*, (\d)>", n) for n in names) if mt), None)
+        if form is not None:
+            break
+    assert form == ("1" if own else "0"), names         # the kernel's last template argument
     assert capi.read_status(reset=True)[0] == 0
-    err = (hidden.float() - want.float()).norm(dim=1) / want.float().norm(dim=1)
+    err = (got.float() - want.float()).norm(dim=1) / want.float().norm(dim=1)
     assert float(err.max()) <= 2e-2
