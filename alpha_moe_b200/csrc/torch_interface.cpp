@@ -112,7 +112,7 @@ void fused_experts(const torch::Tensor& hidden, const torch::Tensor& w1, const t
         TORCH_CHECK((i < 4 ? *weights[i] : i == 4 ? topk_weights : topk_ids).device() == hidden.device(), names[i],
                     " must be on ", hidden.device());
 
-    TORCH_CHECK(block_m > 0, "bad block_m ", block_m);
+    TORCH_CHECK(block_m > 0, "alpha_moe_b200 error ", ALPHA_MOE_E_ARG, ": bad block_m ", block_m);     // (sizes the scratch below)
 
     const c10::cuda::CUDAGuard device_guard(hidden.device());
     const cudaStream_t stream = at::cuda::getCurrentCUDAStream();

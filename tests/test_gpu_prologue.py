@@ -499,6 +499,9 @@ def test_layer_call_refuses_cuda_tensors_in_the_words_of_the_host_checks():
             call(knobs)
     with pytest.raises(capi.AlphaMoeError, match="stages"):
         call(dict(conf, stages=9, block_m=128, block_n=64, warp_n=4))
+    for block_m in (-8, 0, 12, 136):
+        with pytest.raises(capi.AlphaMoeError, match="bad block_m"):
+            call(dict(conf, block_m=block_m))
     assert bool((good["hidden_states"] == 1).all())
     # other dtypes and layouts of the routing are converted; a buffer that requires gradients is overwritten all the same
     out = call(topk_ids=torch.zeros(top_k, m, dtype=torch.int64, device="cuda").t(),
