@@ -1,8 +1,6 @@
 """GPU tests of the two pre-operator kernels, bit-exact against the CPU restatement (integer and
 byte work): block schedule and per-token-group fp8 quantisation, then the whole call-site sequence
 of extra/sglang.patch:25-41 end to end."""
-import re
-
 import pytest
 import torch
 
@@ -589,10 +587,9 @@ def test_layer_call_inside_a_traced_function():
     (33, 9, 40, 256, 40, 64, 3, False),
     (33, 9, 871, 128, 16, 32, 3, False),         # more experts than the histogram has room for
 ])
-def test_which_layer_calls_make_their_own_schedule(m, top_k, e, inter, bm, bn, stages, own):
+def test_which_layer_calls_make_their_own_schedule(m, top_k, e, inter, bm, bn, stages, own, tmp_path):
     """Both sides of every line between the operator that makes its own schedule and the schedule kernel, each against the steps
     one by one, token by token."""
-    from torch.profiler import ProfilerActivity, profile
     from alpha_moe_b200 import capi
     from alpha_moe_b200.layer import fused_experts_impl
     from alpha_moe_b200.prologue import moe_align_block_size, per_token_group_quant_fp8
@@ -610,17 +607,16 @@ def test_which_layer_calls_make_their_own_schedule(m, top_k, e, inter, bm, bn, s
     sid, eid, npp = moe_align_block_size(ids, bm, e)
     want = torch.zeros_like(hidden)
     torch.ops.alpha_moe.fused_moe_w8a8_up_down(xq, xs, w, ws, w2, w2s, sid, eid, npp, wts, want, top_k, bm, bn, 256 // bn, stages, 1.0)
-    form = None
-    for _ in range(4):                       # (the profiler loses a kernel's record now and then)
-        got = hidden.clone()
-        with profile(activities=[ProfilerActivity.CUDA]) as prof:
-            fused_experts_impl(got, w, ws, w2, w2s, wts, ids, config=conf)
-            torch.cuda.synchronize()
-        names = [ev.key for ev in prof.key_averages()]
-        form = next((mt.group(1) for mt in (re.search(r"sm100_kernel<.*, (\d)>", n) for n in names) if mt), None)
-        if form is not None:
-            break
-    assert form == ("1" if own else "0"), names         # the kernel's last template argument
+    got = hidden.clone()
+    fused_experts_impl(got, w, ws, w2, w2s, wts, ids, config=conf)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    graph.enable_debug_mode()
+    with torch.cuda.graph(graph):
+        fused_experts_impl(hidden, w, ws, w2, w2s, wts, ids, config=conf)
+    graph.debug_dump(str(tmp_path / "graph.dot"))         # the launches' names
+    names = (tmp_path / "graph.dot").read_text()
+    assert "fused_moe" in names and ("group_quant" in names or "quant_and_align" in names)
+    assert ("align" in names) != own
     assert capi.read_status(reset=True)[0] == 0
     err = (got.float() - want.float()).norm(dim=1) / want.float().norm(dim=1)
     assert float(err.max()) <= 2e-2
